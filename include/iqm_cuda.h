@@ -45,15 +45,10 @@ typedef struct iqm_ctx iqm_ctx;
 
 typedef enum {
     IQM_FP32 = 0,       /* plain FP32 arithmetic, FP64 pooling sums                              */
-    IQM_MIXED = 1,      /* FSIM: inverse transforms on the tensor cores as FP16 tiles with
-                           split-precision (hi + lo) products and FP32 accumulation, FP16
-                           intermediate planes; FP64 noise threshold and pooling as in IQM_FP32.
-                           Plane sizes without tensor-core engines (all but 480x270, the plane of
-                           1080p and 4K pairs) run the FP32 transforms.
-                           SSIM: the Gaussian window sums on the tensor cores, moments staged as
+    IQM_MIXED = 1,      /* SSIM: the Gaussian window sums on the tensor cores, moments staged as
                            FP16 hi + lo pairs, split-precision products, FP32 accumulation.
-                           Scores within 1e-4 of the FP64 oracle.  FLIP and M-SVD compute in FP32
-                           whatever is asked.                                                      */
+                           Scores within 1e-4 of the FP64 oracle.  FSIM, FLIP and M-SVD compute in
+                           FP32 whatever is asked.                                                 */
     IQM_MIXED_FAST = 2  /* as IQM_MIXED with single FP16 operands and products (hi parts only)  */
 } iqm_precision;
 

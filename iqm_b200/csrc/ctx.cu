@@ -51,6 +51,7 @@ extern "C" __attribute__((visibility("default"))) int iqm_create(int device, iqm
 
 void iqm_release_fsim_plans(iqm_ctx *ctx);  // fsim.cu
 void iqm_release_fft_plans(iqm_ctx *ctx);   // fft.cu
+void iqm_release_reg_plans(iqm_ctx *ctx);   // fft_reg.cu
 
 extern "C" __attribute__((visibility("default"))) int iqm_destroy(iqm_ctx *ctx) {
     if (!ctx) return IQM_EINVAL;
@@ -58,6 +59,7 @@ extern "C" __attribute__((visibility("default"))) int iqm_destroy(iqm_ctx *ctx) 
     cudaStreamSynchronize(ctx->stream);
     iqm_release_fsim_plans(ctx);
     iqm_release_fft_plans(ctx);
+    iqm_release_reg_plans(ctx);
     ctx->desc.release();
     ctx->scratch.release();
     ctx->images.release();

@@ -8,14 +8,12 @@
 //
 // Here, per group of pairs with the same W'xH', seven kernels:
 //   fsim_ingest_kernel      full-resolution RGBA8 -> I, Q, Y planes of both images (box F x F)
-//   fsim_fwd_rows_kernel    forward FFT along x of a pair's two luma planes packed as one complex
-//                           plane Y_img + i Y_ref (shared-memory Stockham)
-//   fsim_fwd_cols_kernel    forward FFT along y
-//   fsim_inv_cols_kernel    each image's spectrum separated from the packed one (Hermitian halves),
-//                           x log-Gabor_s x angular_o, inverse FFT along y (32 planes)
-//   fsim_inv_rows_kernel    inverse FFT along x of the 4 scales of one orientation, scaled 1/N,
-//                           fused with the response sums of fsim_sum_filter_responses.glsl and
-//                           the |EO(s=0)|^2 values of fsim_pack_for_median.glsl
+//   forward rows, columns   FFT of a pair's two luma planes packed as one complex plane
+//                           Y_img + i Y_ref, then each image's own spectrum (Hermitian halves)
+//   inverse columns         spectrum x log-Gabor_s x angular_o, inverse FFT along y (32 planes)
+//   inverse rows            inverse FFT along x of the 4 scales of one orientation, normalised, fused
+//                           with the response sums of fsim_sum_filter_responses.glsl and the
+//                           |EO(s=0)|^2 values of fsim_pack_for_median.glsl
 //   fsim_noise_kernel       exact upper median by radix select (no host round trip), noise power
 //                           and the phase-congruency threshold T in FP64
 //   fsim_final_kernel       phase congruency, gradient (3x3 on the fly), similarity terms and the
@@ -23,9 +21,14 @@
 // The 16 filters and the size-only constants (EM_n, EstSumAn2, EstSumAiAj; fsim_filter_noise.glsl,
 // fsim_mult_filters.glsl) are built once per W'xH' with the same kernels and cached on the context.
 // Schedule per group: ingest and the forward transform for all pairs at once; the two inverse passes
-// in chunks of pairs whose 32 intermediate planes fit the 126 MB L2; noise and final kernels for
-// all pairs at once.  Every transform runs on one warp (fft.cuh warp engine), CTAs hold 1-8 of
-// them, so stages synchronise with __syncwarp only.
+// in chunks of pairs (chunk_pairs); noise and final kernels for all pairs at once.
+//
+// The transform passes run on the register FFT engine (fft_reg.cuh, fsim_reg_*.cu) whatever the form
+// asked for: its FP32 transforms took 27.0 us a 1080p pair for both inverse passes where FP16 tensor-core
+// transforms took 45 us with split products and 28 us with single ones, so the mixed forms have no
+// transforms of their own.  Planes with a side that engine has no plan for (some lengths above 3000) run
+// on the shared-memory engine of fft.cuh, in the kernels of this file: one warp per transform, or a whole
+// CTA where per-warp buffers would leave few warps per SM.
 #include <algorithm>
 #include <cmath>
 #include <initializer_list>
@@ -33,67 +36,66 @@
 #include <mutex>
 #include <tuple>
 
-#include "dft_mma.cuh"
 #include "fft.cuh"
 #include "fft_plan.cuh"
+#include "fft_reg_plan.cuh"
+#include "fsim_internal.cuh"
+#include "fsim_reg.cuh"
 #include "iqm_internal.cuh"
 #include "select.cuh"
 
 #define GLSL_PI 3.141592653589
 
 namespace iqm {
-
-struct FsimPlan {
-    int w2 = 0, h2 = 0, n = 0;
-    FftLen row{}, col{};
-    float *filters = nullptr;  // 16 planes of n (z = o*4 + s)
-    double *consts = nullptr;  // device: em[4], an2[2][4], aiaj[2][4]
-    void *mma_tables = nullptr;  // tensor-core engines' constants (480 x 270 plans in a mixed form)
-    double em[4], an2[2][4], aiaj[2][4];
-    ~FsimPlan() {
-        if (filters) cudaFree(filters);
-        if (consts) cudaFree(consts);
-        if (mma_tables) cudaFree(mma_tables);
+// Raises a kernel's dynamic shared-memory limit on the current device to at least `bytes` (never
+// lowers it: launches already enqueued or captured for other plane sizes keep their sizes valid).
+void set_smem(const void *fn, size_t bytes, bool carveout) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> current;  // kernel attributes are per device
+    int dev = 0;
+    IQM_CHECK_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_pair(dev, fn);
+    auto it = current.find(key);
+    if (it == current.end()) {
+        // shared-memory bound CTAs: the largest carveout, so that as many fit per SM as registers allow
+        if (carveout) IQM_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        it = current.emplace(key, 0).first;
     }
-};
+    if (bytes <= 48 * 1024 || bytes <= it->second) return;
+    IQM_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+    it->second = bytes;
+}
+
+int resident_ctas(const void *fn, int threads, size_t smem, bool carveout) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, const void *, int, size_t>, int> known;
+    int dev = 0;
+    IQM_CHECK_CUDA(cudaGetDevice(&dev));
+    const auto key = std::make_tuple(dev, fn, threads, smem);
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        auto it = known.find(key);
+        if (it != known.end()) return it->second;
+    }
+    set_smem(fn, smem, carveout);
+    int blocks = 0;
+    IQM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, threads, smem));
+    std::lock_guard<std::mutex> lock(mu);
+    known[key] = blocks;
+    return blocks;
+}
 
 }  // namespace iqm
 
 using iqm::FftLen;
+using iqm::set_smem;
+using iqm::FsimGroup;
+using iqm::FsimPairDev;
+using iqm::FT;
+using iqm::response_sums;
 
 namespace {
-
-constexpr int FT = 256;  // threads per FFT / pointwise CTA
-
-struct FsimPairDev {
-    const uint8_t *a;
-    const uint8_t *b;
-    long long pitch;
-    int w, h, F;
-    int out;  // index of this pair in the caller's score array
-};
-
-struct FsimGroup {
-    const FsimPairDev *pairs;
-    int G;          // pairs in this launch
-    int pair0;      // group index of the first pair of this launch (inverse-pass chunks)
-    int w2, h2, n;
-    float *yiq;     // G x 2 x 3 x n   (I, Q, Y)
-    float2 *spec;   // G x n: per pair the spectrum of Y_img + i Y_ref
-    float2 *T;      // chunk x 2 x 16 x n  (after the column pass of the inverse transform)
-    __half2 *Th;    // the same planes in FP16 (mixed precision; shares T's memory)
-    float *amp;     // G x 8 x n       (img*4 + o)
-    float *energy;  // G x 8 x n
-    float *eo0;     // G x 8 x n       |EO(s=0, o)|^2
-    float *thr;     // G x 8
-    double *partials;  // G x tiles x 3
-    unsigned *counters;
-    int tiles;
-    double *scores;    // 2 per pair: fsim, fsimc
-    const float *filters;  // 16 planes, column-major: filters[z][x * h2 + y]
-    const double *consts;
-    int energy_mode;
-};
 
 // ---------------------------------------------------------------------------------------------
 // filters -- shaders/fsim/fsim_lowpassfilter.glsl:21-42 (cutoff 0.45, order 15),
@@ -104,7 +106,9 @@ __device__ __forceinline__ float freq_coord(int i, int n) {
     return float(shifted - n / 2) / float(n);
 }
 
-__global__ void fsim_filters_kernel(float *filters, int w2, int h2) {
+// tile != 0 (register engine): planes of `tiled` elements in tiles of 2^lc columns (FsimPlan), divided by
+// the plane's N points so that the inverse transforms come out normalised; else column-major and unscaled.
+__global__ void fsim_filters_kernel(float *filters, int w2, int h2, int lc, int tile, int tiled) {
     const int n = w2 * h2;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
@@ -133,18 +137,26 @@ __global__ void fsim_filters_kernel(float *filters, int w2, int h2) {
         const float dtheta = fabsf(atan2f(ds, dc));
         const float a = expf(-(dtheta * dtheta) / (2.0f * (theta_sigma * theta_sigma)));
 #pragma unroll
-        for (int s = 0; s < 4; s++) filters[(o * 4 + s) * n + x * h2 + y] = lg[s] * a;
+        for (int s = 0; s < 4; s++) {
+            const float v = lg[s] * a;
+            if (tile)
+                filters[size_t(o * 4 + s) * tiled + (x >> lc) * tile + (y << lc) + (x & ((1 << lc) - 1))] = v / float(n);
+            else
+                filters[size_t(o * 4 + s) * n + x * h2 + y] = v;
+        }
     }
 }
 
-// EM_n(o) = sum_p H[o*4+0](p)^2 (fsim_filter_combinations.cpp:76-134 with fsim_filter_noise.glsl)
-__global__ void fsim_em_kernel(const float *filters, int n, double *consts) {
+// EM_n(o) = sum_p H[o*4+0](p)^2 (fsim_filter_combinations.cpp:76-134 with fsim_filter_noise.glsl);
+// filters as fsim_filters_kernel wrote them.
+__global__ void fsim_em_kernel(const float *filters, int w2, int h2, int lc, int tile, int tiled, double *consts) {
     __shared__ double red[FT / 32];
-    const int o = blockIdx.x;
-    const float *f = filters + (o * 4) * n;
+    const int o = blockIdx.x, n = w2 * h2;
+    const float *f = filters + size_t(o * 4) * (tile ? tiled : n);
     double s = 0.0;
     for (int p = threadIdx.x; p < n; p += FT) {
-        const float v = f[p];
+        const int x = p % w2, y = p / w2;
+        const float v = tile ? float(double(f[(x >> lc) * tile + (y << lc) + (x & ((1 << lc) - 1))]) * n) : f[x * h2 + y];
         s += double(v * v);
     }
     for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
@@ -257,68 +269,14 @@ __global__ void __launch_bounds__(FT) fsim_ingest_kernel(FsimGroup g) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Transform kernels.  Shared memory of every transform CTA starts with the stage twiddles of its
+// Transform kernels of the shared-memory engine.  Shared memory of every transform CTA starts with the stage twiddles of its
 // length (FftLen::stw), followed by per-warp work buffers: a warp transforms NB sequences at once in
-// buffer a (NB x wl) and, unless the engine transforms in place, a ping-pong buffer b of the same
-// size.
+// buffer a (NB x wl) and a ping-pong buffer b of the same size.
 constexpr int NB = 1;  // the transform engines run one sequence per warp
 static_assert(NB == 1, "column slabs index with cols == 1 << lw");
 
-
-// Transform engines: the runtime-planned warp engine for any length, or a fixed-length one whose
-// radix sequence is compiled in (the host picks it only when it equals the length's own plan, so
-// the stage twiddle table in shared memory has the layout it expects).
-struct GenericEngine {
-    static __device__ __forceinline__ float2 *run(float2 *a, float2 *b, const FftLen &L, const float2 *stw, float s,
-                                                  int wl) {
-        return iqm::fft_warp(a, b, L, stw, s, 1, wl);
-    }
-};
-template <class FP>
-struct FixedEngine {
-    static __device__ __forceinline__ float2 *run(float2 *a, float2 *b, const FftLen &, const float2 *stw, float s,
-                                                  int) {
-        return FP::run(a, b, stw, s);
-    }
-};
-// Transform length an engine is compiled for (0: any length).
-template <class E>
-struct engine_len {
-    static constexpr int value = 0;
-};
-template <class FP>
-struct engine_len<FixedEngine<FP>> {
-    static constexpr int value = FP::n;
-};
-
-// Work buffers a transform needs: two for the ping-pong engines, one for the in-place fixed plans.
-template <class FP>
-struct plan_bufs {
-    static constexpr int value = 2;
-};
-template <int N, int... Rs>
-struct plan_bufs<iqm::FixedPlanIP<N, Rs...>> {
-    static constexpr int value = 1;
-};
-template <class E>
-struct engine_bufs {
-    static constexpr int value = 2;
-};
-template <class FP>
-struct engine_bufs<FixedEngine<FP>> {
-    static constexpr int value = plan_bufs<FP>::value;
-};
-
-// The work area of warp `warp` in a CTA whose warps each hold engine_bufs<E> buffers of wl points.
-template <class E>
-__device__ __forceinline__ float2 *warp_area(float2 *base, int warp, int wl) {
-    return base + size_t(warp) * engine_bufs<E>::value * NB * wl;
-}
-
-// 480 (the row length, whose pass is limited by shared memory) transforms in place; 270 (the column
-// length, whose pass is limited by registers) keeps the two-buffer form.
-using Engine270 = FixedEngine<iqm::FixedPlan<270, 9, 3, 10>>;
-using Engine480 = FixedEngine<iqm::FixedPlanIP<480, 15, 8, 4>>;
+// The work area of warp `warp` in a CTA whose warps each hold two buffers of wl points.
+__device__ __forceinline__ float2 *warp_area(float2 *base, int warp, int wl) { return base + size_t(warp) * 2 * NB * wl; }
 
 // Strided copy with up to 8 independent loads in flight per thread: ld(i) for i = first, first +
 // step, ... < n, in batches of 8 loads before their 8 stores st(i, v) (runtime-length paths, whose
@@ -341,9 +299,7 @@ struct F2x2 {
 
 // forward transform (src/gpu/fsim/fsim.cpp:270-368: luma as complex (Y, 0), sign -1, unscaled),
 // NB rows per warp.
-template <class Eng>
-// Compiled engines: 4 CTAs per SM (62 registers with the 480-point engine, no spills).
-__global__ void __launch_bounds__(FT, engine_len<Eng>::value ? 4 : 1) fsim_fwd_rows_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl) {
+__global__ void __launch_bounds__(FT, 1) fsim_fwd_rows_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl) {
     extern __shared__ __align__(16) float2 sm[];
     const int tl = iqm::stage_twiddle_len(L);
     iqm::stage_twiddles_to_shared(L, sm);
@@ -355,30 +311,15 @@ __global__ void __launch_bounds__(FT, engine_len<Eng>::value ? 4 : 1) fsim_fwd_r
     const int y0 = (blockIdx.x * (blockDim.x >> 5) + warp) * NB;
     if (y0 >= g.h2) return;  // warp-uniform; no block-wide barrier follows
     const int nb = min(NB, g.h2 - y0);
-    float2 *a = warp_area<Eng>(work, warp, wl), *b = a + NB * wl;
+    float2 *a = warp_area(work, warp, wl), *b = a + NB * wl;
     const float *Y1 = g.yiq + (size_t(pair * 2) * 3 + 2) * g.n + size_t(y0) * g.w2;
     const float *Y2 = Y1 + size_t(3) * g.n;  // the pair's second image
-    constexpr int PN = engine_len<Eng>::value;
     for (int t = 0; t < nb; t++) {
-        if constexpr (PN > 0) {  // fixed length: the row's loads all in flight before the stores
-            constexpr int PV = (PN + 31) / 32;
-            float v1[PV], v2[PV];
-#pragma unroll
-            for (int i = 0; i < PV; i++)
-                if (lane + 32 * i < PN) {
-                    v1[i] = __ldcg(Y1 + size_t(t) * g.w2 + lane + 32 * i);
-                    v2[i] = __ldcg(Y2 + size_t(t) * g.w2 + lane + 32 * i);
-                }
-#pragma unroll
-            for (int i = 0; i < PV; i++)
-                if (lane + 32 * i < PN) a[t * wl + lane + 32 * i] = make_float2(v1[i], v2[i]);
-        } else {
-            batched_copy<float2>(
-                lane, g.w2, 32, [&](int x) { return make_float2(Y1[size_t(t) * g.w2 + x], Y2[size_t(t) * g.w2 + x]); },
-                [&](int x, float2 v) { a[t * wl + x] = v; });
-        }
+        batched_copy<float2>(
+            lane, g.w2, 32, [&](int x) { return make_float2(Y1[size_t(t) * g.w2 + x], Y2[size_t(t) * g.w2 + x]); },
+            [&](int x, float2 v) { a[t * wl + x] = v; });
     }
-    const float2 *res = Eng::run(a, b, L, sm, -1.f, wl);
+    const float2 *res = iqm::fft_warp(a, b, L, sm, -1.f, 1, wl);
     float2 *S = g.spec + size_t(pair) * g.n + size_t(y0) * g.w2;
     for (int t = 0; t < nb; t++)
         for (int x = lane; x < g.w2; x += 32) S[size_t(t) * g.w2 + x] = res[t * wl + x];
@@ -388,10 +329,7 @@ __global__ void __launch_bounds__(FT, engine_len<Eng>::value ? 4 : 1) fsim_fwd_r
 // is loaded and stored cooperatively and each warp transforms NB of its columns.
 __device__ __forceinline__ int slab_parity(float2 *res, float2 *a) { return res == a ? 0 : 1; }
 
-template <class Eng>
-// Compiled engines: 5 CTAs per SM with the two-buffer 270-point engine (48 registers), 4 with the
-// in-place 480-point one (63 registers); no spills either way.
-__global__ void __launch_bounds__(FT, engine_len<Eng>::value ? (engine_bufs<Eng>::value == 2 ? 5 : 4) : 1)
+__global__ void __launch_bounds__(FT, 1)
 fsim_fwd_cols_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl, int lw) {
     extern __shared__ __align__(16) float2 sm[];
     __shared__ int parity;
@@ -404,45 +342,27 @@ fsim_fwd_cols_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl, int 
     const int nc = min(cols, g.w2 - x0);
     float2 *S = g.spec + size_t(pair) * g.n;
     // column c lives in warp c / NB, slot c % NB
-    constexpr int PN = engine_len<Eng>::value;
-    if constexpr (PN > 0) {  // fixed length: each thread's slab loads all in flight before the stores
-        constexpr int KS = (NB * PN + 31) / 32;
-        float2 v[KS];
-#pragma unroll
-        for (int k = 0; k < KS; k++) {
-            const int idx = threadIdx.x + k * blockDim.x;
+    batched_copy<float2>(
+        threadIdx.x, cols * g.h2, blockDim.x,
+        [&](int idx) {
             const int c = idx & (cols - 1), y = idx >> lw;  // cols = 1 << lw
-            if (idx < cols * g.h2 && c < nc) v[k] = __ldcg(S + size_t(y) * g.w2 + x0 + c);
-        }
-#pragma unroll
-        for (int k = 0; k < KS; k++) {
-            const int idx = threadIdx.x + k * blockDim.x;
+            return c < nc ? S[size_t(y) * g.w2 + x0 + c] : make_float2(0.f, 0.f);
+        },
+        [&](int idx, float2 v) {
             const int c = idx & (cols - 1), y = idx >> lw;
-            if (idx < cols * g.h2 && c < nc) warp_area<Eng>(work, c / NB, wl)[(c % NB) * wl + y] = v[k];
-        }
-    } else {
-        batched_copy<float2>(
-            threadIdx.x, cols * g.h2, blockDim.x,
-            [&](int idx) {
-                const int c = idx & (cols - 1), y = idx >> lw;  // cols = 1 << lw
-                return c < nc ? S[size_t(y) * g.w2 + x0 + c] : make_float2(0.f, 0.f);
-            },
-            [&](int idx, float2 v) {
-                const int c = idx & (cols - 1), y = idx >> lw;
-                if (c < nc) warp_area<Eng>(work, c / NB, wl)[(c % NB) * wl + y] = v;
-            });
-    }
+            if (c < nc) warp_area(work, c / NB, wl)[(c % NB) * wl + y] = v;
+        });
     __syncthreads();
     const int nbw = min(NB, nc - warp * NB);
     if (nbw > 0) {
-        float2 *a = warp_area<Eng>(work, warp, wl);
-        float2 *res = Eng::run(a, a + NB * wl, L, sm, -1.f, wl);
+        float2 *a = warp_area(work, warp, wl);
+        float2 *res = iqm::fft_warp(a, a + NB * wl, L, sm, -1.f, 1, wl);
         if (warp == 0 && (threadIdx.x & 31) == 0) parity = slab_parity(res, a);
     }
     __syncthreads();
     for (int idx = threadIdx.x; idx < cols * g.h2; idx += blockDim.x) {
         const int c = idx & (cols - 1), y = idx >> lw;  // cols = 1 << lw
-        if (c < nc) S[size_t(y) * g.w2 + x0 + c] = warp_area<Eng>(work, c / NB, wl)[parity * NB * wl + (c % NB) * wl + y];
+        if (c < nc) S[size_t(y) * g.w2 + x0 + c] = warp_area(work, c / NB, wl)[parity * NB * wl + (c % NB) * wl + y];
     }
 }
 
@@ -450,10 +370,7 @@ fsim_fwd_cols_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl, int 
 // inverse transform, pass 1 (along y) of the 4 filtered spectra of orientation o:
 // spectrum x H[o*4+s] (fsim_filter_combinations.glsl:53-56), sign +1.  consts_mode uses a
 // spectrum of ones, i.e. transforms the filters themselves (block 0 of the reference's buffer).
-template <class Eng>
-// Two-buffer compiled engines: 4 CTAs per SM (64 registers; with the largest shared-memory carveout
-// the work buffers of 4 CTAs fit).  The runtime-planned and in-place engines need more registers here.
-__global__ void __launch_bounds__(FT, engine_len<Eng>::value && engine_bufs<Eng>::value == 2 ? 4 : 1)
+__global__ void __launch_bounds__(FT, 1)
 fsim_inv_cols_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl, int lw, int consts_mode) {
     extern __shared__ __align__(16) float2 sm[];
     __shared__ int parity;
@@ -470,100 +387,47 @@ fsim_inv_cols_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl, int 
     const int img = plane & 1;
     const float2 *src = g.spec + size_t(g.pair0 + (plane >> 1)) * g.n;  // the pair's packed spectrum
     const int nbw = min(NB, nc - warp * NB);
-    // With a fixed-length engine (h2 == PN) each lane holds its share of the warp's filter column in
-    // registers, and the next scale's share is loaded while this scale's transform runs.
-    constexpr int PN = engine_len<Eng>::value;
-    constexpr int PV = PN > 0 ? (PN + 31) / 32 : 1;
-    float hnext[PV];
-    auto load_filter = [&](int zz) {
-        const float *H = g.filters + size_t(zz) * g.n + size_t(x0 + warp) * h2;
-#pragma unroll
-        for (int i = 0; i < PV; i++) {
-            const int y = lane + 32 * i;
-            hnext[i] = (y < PN) ? __ldg(H + y) : 0.f;
-        }
-    };
-    if (PN > 0 && nbw > 0) load_filter(o * 4);
     // Z = F(Y_img + i Y_ref): F(Y_img) = (Z(k) + conj Z(-k)) / 2, F(Y_ref) = (Z(k) - conj Z(-k)) / 2i
     auto separate = [&](float2 z, float2 m) {
         return img == 0 ? make_float2(0.5f * (z.x + m.x), 0.5f * (z.y - m.y))
                         : make_float2(0.5f * (z.y + m.y), 0.5f * (m.x - z.x));
     };
-    if constexpr (PN > 0) {
-        // fixed length: each thread's NB * PN / 32 slab entries, all loads in flight before the stores
-        // (blockDim.x = 32 nw threads cover cols * PN = NB nw PN entries)
-        constexpr int KS = (NB * PN + 31) / 32;
-        float2 zv[KS], mv[KS];
-#pragma unroll
-        for (int k = 0; k < KS; k++) {
-            const int idx = threadIdx.x + k * blockDim.x;
+    batched_copy<F2x2>(
+        threadIdx.x, cols * h2, blockDim.x,
+        [&](int idx) {
             const int c = idx & (cols - 1), y = idx >> lw;  // cols = 1 << lw
-            zv[k] = mv[k] = make_float2(1.f, 0.f);
-            if (idx < cols * h2 && c < nc && !consts_mode) {
+            F2x2 p{make_float2(1.f, 0.f), make_float2(1.f, 0.f)};
+            if (c < nc && !consts_mode) {
                 const int x = x0 + c;
-                zv[k] = __ldcg(src + size_t(y) * g.w2 + x);
-                mv[k] = __ldcg(src + size_t(y ? h2 - y : 0) * g.w2 + (x ? g.w2 - x : 0));
+                p.z = src[size_t(y) * g.w2 + x];
+                p.m = src[size_t(y ? h2 - y : 0) * g.w2 + (x ? g.w2 - x : 0)];
             }
-        }
-#pragma unroll
-        for (int k = 0; k < KS; k++) {
-            const int idx = threadIdx.x + k * blockDim.x;
+            return p;
+        },
+        [&](int idx, F2x2 p) {
             const int c = idx & (cols - 1), y = idx >> lw;
-            if (idx < cols * h2 && c < nc) Sl[size_t(c) * h2 + y] = consts_mode ? make_float2(1.f, 0.f) : separate(zv[k], mv[k]);
-        }
-    } else {
-        batched_copy<F2x2>(
-            threadIdx.x, cols * h2, blockDim.x,
-            [&](int idx) {
-                const int c = idx & (cols - 1), y = idx >> lw;  // cols = 1 << lw
-                F2x2 p{make_float2(1.f, 0.f), make_float2(1.f, 0.f)};
-                if (c < nc && !consts_mode) {
-                    const int x = x0 + c;
-                    p.z = src[size_t(y) * g.w2 + x];
-                    p.m = src[size_t(y ? h2 - y : 0) * g.w2 + (x ? g.w2 - x : 0)];
-                }
-                return p;
-            },
-            [&](int idx, F2x2 p) {
-                const int c = idx & (cols - 1), y = idx >> lw;
-                if (c < nc) Sl[size_t(c) * h2 + y] = consts_mode ? make_float2(1.f, 0.f) : separate(p.z, p.m);
-            });
-    }
+            if (c < nc) Sl[size_t(c) * h2 + y] = consts_mode ? make_float2(1.f, 0.f) : separate(p.z, p.m);
+        });
     __syncthreads();
     for (int s = 0; s < 4; s++) {
         const int z = o * 4 + s;
         if (nbw > 0) {
-            float2 *a = warp_area<Eng>(work, warp, wl);
+            float2 *a = warp_area(work, warp, wl);
             const float2 *col = Sl + size_t(warp) * h2;  // NB == 1: column `warp` of the slab
-            if constexpr (PN > 0) {
-                float hcur[PV];
-#pragma unroll
-                for (int i = 0; i < PV; i++) hcur[i] = hnext[i];
-                if (s < 3) load_filter(z + 1);
-#pragma unroll
-                for (int i = 0; i < PV; i++) {
-                    const int y = lane + 32 * i;
-                    if (y < PN) {
-                        const float2 v = col[y];
-                        a[y] = make_float2(hcur[i] * v.x, hcur[i] * v.y);
-                    }
-                }
-            } else {
-                const float *H = g.filters + size_t(z) * g.n + size_t(x0 + warp) * h2;
-                for (int y = lane; y < h2; y += 32) {
-                    const float hv = __ldg(H + y);
-                    const float2 v = col[y];
-                    a[y] = make_float2(hv * v.x, hv * v.y);
-                }
+            const float *H = g.filters + size_t(z) * g.n + size_t(x0 + warp) * h2;
+            for (int y = lane; y < h2; y += 32) {
+                const float hv = __ldg(H + y);
+                const float2 v = col[y];
+                a[y] = make_float2(hv * v.x, hv * v.y);
             }
-            float2 *res = Eng::run(a, a + NB * wl, L, sm, 1.f, wl);
+            float2 *res = iqm::fft_warp(a, a + NB * wl, L, sm, 1.f, 1, wl);
             if (warp == 0 && lane == 0) parity = slab_parity(res, a);
         }
         __syncthreads();
         float2 *dst = g.T + (size_t(plane) * 16 + z) * g.n;
         for (int idx = threadIdx.x; idx < cols * h2; idx += blockDim.x) {
             const int c = idx & (cols - 1), y = idx >> lw;  // cols = 1 << lw
-            if (c < nc) dst[size_t(y) * g.w2 + x0 + c] = warp_area<Eng>(work, c / NB, wl)[parity * NB * wl + (c % NB) * wl + y];
+            if (c < nc) dst[size_t(y) * g.w2 + x0 + c] = warp_area(work, c / NB, wl)[parity * NB * wl + (c % NB) * wl + y];
         }
         __syncthreads();
     }
@@ -621,34 +485,12 @@ fsim_inv_cols_seq_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl, 
     }
 }
 
-// Per-pixel response sums of one orientation from its 4 scales (scaled by 1/N here), as
-// shaders/fsim/fsim_sum_filter_responses.glsl:43-80 and fsim_pack_for_median.glsl:39-43; square
-// roots and the reciprocal from the SFU approximations.
-__device__ __forceinline__ void response_sums(const float2 v[4], float invN, float &sA, float &en, float &e0) {
-    float re[4], im[4];
-    float sE = 0.f, sO = 0.f;
-    sA = 0.f;
-#pragma unroll
-    for (int s = 0; s < 4; s++) {
-        re[s] = v[s].x * invN;
-        im[s] = v[s].y * invN;
-        sA += iqm::sqrt_nonneg(re[s] * re[s] + im[s] * im[s]);
-        sE += re[s];
-        sO += im[s];
-    }
-    const float rxe = iqm::rcp_approx(iqm::sqrt_nonneg(sE * sE + sO * sO) + 0.0001f);
-    const float mE = sE * rxe, mO = sO * rxe;
-    en = 0.f;
-#pragma unroll
-    for (int s = 0; s < 4; s++) en += re[s] * mE + im[s] * mO - fabsf(re[s] * mO - im[s] * mE);
-    e0 = re[0] * re[0] + im[0] * im[0];
-}
+__device__ __forceinline__ float2 scaled(float2 v, float s) { return make_float2(v.x * s, v.y * s); }
 
 // inverse transform, pass 2 (along x): a CTA handles rr rows with WPR = 4/NB warps per row;
 // warp (r, h) transforms scales h*NB .. h*NB+NB-1 of row y0 + r.  consts_mode (rr = 1) instead accumulates, per row, sum_s Re_s^2 N and
 // sum_{i<j} Re_i Re_j N (shaders/fsim/fsim_mult_filters.glsl:37-58) over p < ceil(N/2) and all p.
-template <class Eng>
-__global__ void __launch_bounds__(FT, engine_len<Eng>::value ? 4 : 1) fsim_inv_rows_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl, int rr, int consts_mode,
+__global__ void __launch_bounds__(FT, 1) fsim_inv_rows_kernel(FsimGroup g, const __grid_constant__ FftLen L, int wl, int rr, int consts_mode,
                                                               double *rowsums) {
     extern __shared__ __align__(16) float2 sm[];
     __shared__ int parity;
@@ -666,33 +508,20 @@ __global__ void __launch_bounds__(FT, engine_len<Eng>::value ? 4 : 1) fsim_inv_r
     {
         const int y = y0 + r;
         if (r < rr && y < g.h2) {
-            float2 *a = warp_area<Eng>(work, warp, wl);
-            constexpr int PN = engine_len<Eng>::value;
-            for (int t = 0; t < NB; t++) {
+            float2 *a = warp_area(work, warp, wl);
+                    for (int t = 0; t < NB; t++) {
                 const float2 *src = g.T + (size_t(plane) * 16 + o * 4 + h * NB + t) * g.n + size_t(y) * w2;
-                if constexpr (PN > 0) {
-                    // fixed length: every load of the row is in flight before the first store
-                    constexpr int PV = (PN + 31) / 32;
-                    float2 v[PV];
-#pragma unroll
-                    for (int i = 0; i < PV; i++)
-                        if (lane + 32 * i < PN) v[i] = __ldcg(src + lane + 32 * i);
-#pragma unroll
-                    for (int i = 0; i < PV; i++)
-                        if (lane + 32 * i < PN) a[t * wl + lane + 32 * i] = v[i];
-                } else {
-                    batched_copy<float2>(lane, w2, 32, [&](int x) { return src[x]; },
-                                         [&](int x, float2 v) { a[t * wl + x] = v; });
-                }
+                batched_copy<float2>(lane, w2, 32, [&](int x) { return src[x]; },
+                                     [&](int x, float2 v) { a[t * wl + x] = v; });
             }
-            float2 *res = Eng::run(a, a + NB * wl, L, sm, 1.f, wl);
+            float2 *res = iqm::fft_warp(a, a + NB * wl, L, sm, 1.f, 1, wl);
             if (warp == 0 && lane == 0) parity = slab_parity(res, a);
         }
     }
     __syncthreads();
     // scale s of row rl: warp rl*WPR + s/NB, slot s%NB
     auto at = [&](int rl, int s, int x) -> float2 {
-        return warp_area<Eng>(work, rl * WPR + s / NB, wl)[parity * NB * wl + (s % NB) * wl + x];
+        return warp_area(work, rl * WPR + s / NB, wl)[parity * NB * wl + (s % NB) * wl + x];
     };
     const float invN = 1.0f / float(g.n);
     if (!consts_mode && (w2 & 3) == 0 && rr <= 2) {
@@ -710,7 +539,7 @@ __global__ void __launch_bounds__(FT, engine_len<Eng>::value ? 4 : 1) fsim_inv_r
             float2 v[4][4];  // [scale][pixel]
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const float4 *src4 = reinterpret_cast<const float4 *>(&warp_area<Eng>(work, rl * WPR + q / NB, wl)[parity * NB * wl + (q % NB) * wl + x]);
+                const float4 *src4 = reinterpret_cast<const float4 *>(&warp_area(work, rl * WPR + q / NB, wl)[parity * NB * wl + (q % NB) * wl + x]);
                 const float4 lo = src4[0], hi = src4[1];
                 v[q][0] = make_float2(lo.x, lo.y);
                 v[q][1] = make_float2(lo.z, lo.w);
@@ -719,8 +548,8 @@ __global__ void __launch_bounds__(FT, engine_len<Eng>::value ? 4 : 1) fsim_inv_r
             }
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const float2 w[4] = {v[0][i], v[1][i], v[2][i], v[3][i]};
-                response_sums(w, invN, pa[i], pe[i], p0[i]);
+                const float2 w[4] = {scaled(v[0][i], invN), scaled(v[1][i], invN), scaled(v[2][i], invN), scaled(v[3][i], invN)};
+                response_sums(w, pa[i], pe[i], p0[i]);
             }
             const size_t off = (size_t(gp) * 4 + o) * g.n + size_t(y) * w2 + x;
             *reinterpret_cast<float4 *>(g.amp + off) = oa;
@@ -736,9 +565,9 @@ __global__ void __launch_bounds__(FT, engine_len<Eng>::value ? 4 : 1) fsim_inv_r
             for (int x = threadIdx.x; x < w2; x += blockDim.x) {
                 float2 v[4];
 #pragma unroll
-                for (int q = 0; q < 4; q++) v[q] = at(rl, q, x);
+                for (int q = 0; q < 4; q++) v[q] = scaled(at(rl, q, x), invN);
                 float sA, en, e0;
-                response_sums(v, invN, sA, en, e0);
+                response_sums(v, sA, en, e0);
                 g.amp[row + x] = sA;
                 g.energy[row + x] = en;
                 g.eo0[row + x] = e0;
@@ -819,9 +648,9 @@ __global__ void __launch_bounds__(FT, 1) fsim_inv_rows_seq_kernel(FsimGroup g, c
         for (int x = threadIdx.x; x < w2; x += FT) {
             float2 v[4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) v[q] = keep[q * w2 + x];
+            for (int q = 0; q < 4; q++) v[q] = scaled(keep[q * w2 + x], invN);
             float sA, en, e0;
-            response_sums(v, invN, sA, en, e0);
+            response_sums(v, sA, en, e0);
             g.amp[off + x] = sA;
             g.energy[off + x] = en;
             g.eo0[off + x] = e0;
@@ -863,192 +692,6 @@ __global__ void __launch_bounds__(FT, 1) fsim_inv_rows_seq_kernel(FsimGroup g, c
         rowsums[(size_t(o) * g.h2 + y) * 4 + threadIdx.x] = t;
     }
 }
-
-// ---------------------------------------------------------------------------------------------
-// Mixed precision (IQM_MIXED, IQM_MIXED_FAST): the inverse passes on the tensor cores.  Each
-// transform is a two-factor DFT computed with FP16 mma.sync tiles and FP32 accumulation
-// (dft_mma.cuh); the spectrum is scaled by 1/N as the column pass loads it, so every FP16 operand
-// and the FP16 intermediate planes between the passes stay in range, and the row pass produces the
-// normalised responses directly.  Both kernels are persistent: each warp builds its transform's
-// constant fragments once and the CTAs stride over (columns or rows, orientation, plane) items.
-
-// Column pass: a work item is MCW adjacent columns of one (orientation, pair); warp c transforms
-// column c of both images for the orientation's 4 scales.  The pair's packed spectrum is read once
-// per item and separated into both images' spectra in a shared slab, each column stored as N1
-// segments of N2 points padded to a stride of SEG (conflict-free loads by the engine's lane
-// pattern); each scale's outputs are staged as FP16 rows of MCW columns and written to the
-// intermediate planes as 16-byte row segments.
-constexpr int MCW = 8;
-template <class Dft>
-struct MmaColGeom {
-    static constexpr int H = Dft::N;                                      // column length
-    static constexpr int SEG = Dft::N2 + ((4 - Dft::N2 % 16) + 16) % 16;  // N2 padded to 4 mod 16
-    static constexpr int SLAB = Dft::N1 * SEG;                            // padded column, float2
-    // staging row stride (half2): MCW columns; odd, so the 32 lanes' scattered output rows
-    // k = g + 15 t (+ const) fall at most 2 to a bank (a multiple of 4 puts them 4 to a bank)
-    static constexpr int SP = 13;
-    static constexpr size_t tables = Dft::smem_bytes;
-    static constexpr size_t slab_bytes = sizeof(float2) * 2 * MCW * SLAB;
-    static constexpr int FLD = (H + 3) & ~3;  // per-warp filter column (floats), 16-byte aligned
-    static constexpr size_t stage_bytes = sizeof(__half2) * 2 * H * SP;
-    static constexpr size_t smem = tables + slab_bytes + stage_bytes + sizeof(float) * MCW * FLD;
-    static_assert(MCW == 8 && tables % 16 == 0 && slab_bytes % 16 == 0, "16-byte aligned slab and staging");
-};
-
-template <class Dft>
-// Single-product engines with shared tables fit 3 CTAs per SM without spills; the others 2.
-__global__ void __launch_bounds__(32 * MCW, Dft::P == 1 && !Dft::kRegs ? 3 : 2)
-    fsim_inv_cols_mma_kernel(FsimGroup g, const void *__restrict__ table, int items) {
-    using Gm = MmaColGeom<Dft>;
-    constexpr int H = Gm::H;
-    extern __shared__ __align__(16) float2 sm[];
-    float2 *Sl = sm + Gm::tables / sizeof(float2);                          // [img][column][SLAB]
-    __half2 *stage = reinterpret_cast<__half2 *>(Sl + 2 * MCW * Gm::SLAB);  // [img][y][SP]
-    const int warp = threadIdx.x >> 5;
-    // this warp's column of the current filter, read once per scale for both images
-    float *fcol = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(stage) + Gm::stage_bytes) + warp * Gm::FLD;
-    Dft dft;
-    dft.load(table, sm);  // complete at the item loop's first barrier
-    const int ngroups = (g.w2 + MCW - 1) / MCW;
-    const float hs = 0.5f / float(g.n);
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const int cg = item % ngroups;
-        const int o = (item / ngroups) & 3;
-        const int pr = item / (ngroups * 4);  // chunk-local pair
-        const int x0 = cg * MCW, nc = min(MCW, g.w2 - x0);
-        const float2 *src = g.spec + size_t(g.pair0 + pr) * g.n;
-        for (int idx = threadIdx.x; idx < MCW * H; idx += blockDim.x) {
-            const int y = idx / MCW, c = idx - y * MCW;
-            float2 v0 = make_float2(0.f, 0.f), v1 = v0;
-            if (c < nc) {
-                const int x = x0 + c;
-                // Z = F(Y_img + i Y_ref): F(Y_img) = (Z(k) + conj Z(-k)) / 2, F(Y_ref) = (Z(k) - conj Z(-k)) / 2i
-                const float2 z = src[size_t(y) * g.w2 + x];
-                const float2 m = src[size_t(y ? H - y : 0) * g.w2 + (x ? g.w2 - x : 0)];
-                v0 = make_float2(hs * (z.x + m.x), hs * (z.y - m.y));
-                v1 = make_float2(hs * (z.y + m.y), hs * (m.x - z.x));
-            }
-            const int si = c * Gm::SLAB + (y / Dft::N2) * Gm::SEG + y % Dft::N2;
-            Sl[si] = v0;
-            Sl[MCW * Gm::SLAB + si] = v1;
-        }
-        __syncthreads();
-#pragma unroll 1
-        for (int s = 0; s < 4; s++) {
-            if (warp < nc) {  // warp-uniform
-                const float *Hz = g.filters + size_t(o * 4 + s) * g.n + size_t(x0 + warp) * H;
-                for (int i = threadIdx.x & 31; i < H; i += 32) fcol[i] = __ldg(Hz + i);
-                __syncwarp();
-#pragma unroll 1
-                for (int img = 0; img < 2; img++) {
-                    const float2 *col = Sl + (img * MCW + warp) * Gm::SLAB;
-                    __half2 *st = stage + img * H * Gm::SP + warp;
-                    dft.run(
-                        [&](int n1, int n2) {
-                            const float h = fcol[Dft::N2 * n1 + n2];
-                            const float2 v = col[n1 * Gm::SEG + n2];
-                            return make_float2(h * v.x, h * v.y);
-                        },
-                        [&](int k, int, float2 v) { st[k * Gm::SP] = __floats2half2_rn(v.x, v.y); });
-                }
-            }
-            __syncthreads();
-            const size_t zoff = size_t(o * 4 + s) * g.n + size_t(x0);
-            if (nc == MCW) {
-                for (int idx = threadIdx.x; idx < 2 * H * 2; idx += blockDim.x) {
-                    const int q = idx & 1, r = idx >> 1;  // r = img * H + y
-                    const int img = r / H, y = r - img * H;
-                    const unsigned *row = reinterpret_cast<const unsigned *>(stage + r * Gm::SP + 4 * q);
-                    const uint4 v = make_uint4(row[0], row[1], row[2], row[3]);
-                    *reinterpret_cast<uint4 *>(g.Th + size_t(2 * pr + img) * 16 * g.n + zoff + size_t(y) * g.w2 + 4 * q) = v;
-                }
-            } else {
-                for (int idx = threadIdx.x; idx < 2 * H * MCW; idx += blockDim.x) {
-                    const int c = idx % MCW, r = idx / MCW;
-                    const int img = r / H, y = r - img * H;
-                    if (c < nc) g.Th[size_t(2 * pr + img) * 16 * g.n + zoff + size_t(y) * g.w2 + c] = stage[r * Gm::SP + c];
-                }
-            }
-            __syncthreads();  // staging rows read before the next scale overwrites them
-        }
-    }
-}
-
-// The 32 bits of an FP16 pair, to go into an MMA operand unchanged.
-__device__ __forceinline__ unsigned h2_word(__half2 h) { return *reinterpret_cast<unsigned *>(&h); }
-
-// Row pass: a work item is one row of one (orientation, plane), taken by one warp on its own: it
-// transforms the row for the 4 scales, reading its FP16 inputs straight from the intermediate
-// planes, parks the first 3 scales' outputs in its own shared slots and keeps the last in
-// registers, then forms the response sums of its outputs (as fsim_inv_rows_kernel does) and
-// stores them; no barrier after the tables are loaded.
-constexpr int MRW = 8;  // warps per CTA of the row pass
-template <class Dft>
-struct MmaRowGeom {
-    static constexpr int W = Dft::N;
-    static constexpr int SLOTS = 2 * Dft::NTC;  // output slots per lane
-    static constexpr size_t tables = Dft::smem_bytes;
-    static constexpr size_t smem = tables + sizeof(float2) * MRW * 3 * SLOTS * 32;
-};
-
-template <class Dft>
-__global__ void __launch_bounds__(32 * MRW, Dft::P == 1 ? 2 : 1)
-    fsim_inv_rows_mma_kernel(FsimGroup g, const void *__restrict__ table, int items) {
-    using Gm = MmaRowGeom<Dft>;
-    constexpr int W = Gm::W, SL = Gm::SLOTS;
-    extern __shared__ __align__(16) float2 sm[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float2 *keep = sm + Gm::tables / sizeof(float2) + size_t(warp) * 3 * SL * 32;  // [scale][slot][lane]
-    Dft dft;
-    dft.load(table, sm);
-    __syncthreads();
-    for (int item = blockIdx.x * MRW + warp; item < items; item += gridDim.x * MRW) {  // warp-uniform
-        const int y = item % g.h2;
-        const int o = (item / g.h2) & 3;
-        const int plane = item / (g.h2 * 4);  // chunk-local pair*2 + img
-        float2 last[SL];
-#pragma unroll 1
-        for (int s = 0; s < 4; s++) {
-            const __half2 *src = g.Th + (size_t(plane) * 16 + o * 4 + s) * g.n + size_t(y) * W;
-            dft.run([&](int n1, int n2) { return h2_word(src[Dft::N2 * n1 + n2]); },
-                    [&](int, int slot, float2 v) {
-                        if (s < 3)
-                            keep[(s * SL + slot) * 32 + lane] = v;
-                        else
-                            last[slot] = v;
-                    });
-        }
-        const size_t row = (size_t(g.pair0 * 2 + plane) * 4 + o) * g.n + size_t(y) * W;
-#pragma unroll
-        for (int slot = 0; slot < SL; slot++) {
-            const int k1 = Dft::slot_k1(slot), k2 = Dft::slot_k2(slot);
-            if (k1 >= Dft::N1 || k2 >= Dft::N2) continue;
-            const int x = k1 + Dft::N1 * k2;
-            const float2 v[4] = {keep[slot * 32 + lane], keep[(SL + slot) * 32 + lane], keep[(2 * SL + slot) * 32 + lane],
-                                 last[slot]};
-            float sA, en, e0;
-            response_sums(v, 1.0f, sA, en, e0);  // already normalised
-            g.amp[row + x] = sA;
-            g.energy[row + x] = en;
-            g.eo0[row + x] = e0;
-        }
-    }
-}
-
-// Builds an engine's constant table (one warp).
-template <class Dft>
-__global__ void mma_table_kernel(void *table) {
-    Dft::build(table, 1.f);
-}
-
-// Tensor-core transform engines of the mixed forms: 270 = 15 x 18 (columns), 480 = 16 x 30 (rows).
-// Single products keep the column engine's stage-C matrix and twiddles in registers (measured 5%
-// faster than the shared table at 1080p); split products keep them in shared memory (registers
-// would spill).
-template <int SPLIT>
-using MmaCol270 = iqm::MmaDft<15, 18, SPLIT, SPLIT == 1>;
-template <int SPLIT>
-using MmaRow480 = iqm::MmaDft<16, 30, SPLIT>;
 
 // sum the per-row constants in row order -> an2[mode][o], aiaj[mode][o]
 __global__ void fsim_consts_reduce_kernel(const double *rowsums, int h2, double *consts) {
@@ -1295,31 +938,10 @@ void plane_size(int w, int h, int F, int &w2, int &h2) {  // src/gpu/fsim/fsim.c
 constexpr size_t SMEM_CAP = 200 * 1024;
 constexpr int kFsimStreams = 8;  // plane-size groups in flight at once
 constexpr bool kOverlapChunks = true;  // rotate inverse-pass chunks over several streams
-// Streams (and L2-sized buffers) the chunks rotate over: two fill each other's partial waves; three
-// measured 2% slower (the third chunk's planes crowd the L2).
+// Streams (and buffers) the chunks rotate over: two fill each other's partial waves; three or four
+// measured the same.
 constexpr int kChunkStreams = 2;
-static_assert(kChunkStreams >= 1 && kChunkStreams <= 8, "chunk streams");
 
-// Raises a kernel's dynamic shared-memory limit on the current device to at least `bytes` (never
-// lowers it: launches already enqueued or captured for other plane sizes keep their sizes valid).
-void set_smem(const void *fn, size_t bytes) {
-    static std::mutex mu;
-    static std::map<std::pair<int, const void *>, size_t> current;  // kernel attributes are per device
-    int dev = 0;
-    IQM_CHECK_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
-    const auto key = std::make_pair(dev, fn);
-    auto it = current.find(key);
-    if (it == current.end()) {
-        // transform CTAs are shared-memory bound: ask for the largest shared-memory carveout so
-        // as many CTAs fit per SM as registers allow
-        IQM_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        it = current.emplace(key, 0).first;
-    }
-    if (bytes <= 48 * 1024 || bytes <= it->second) return;
-    IQM_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-    it->second = bytes;
-}
 
 // Launch shapes of the transform kernels for one plane size.
 struct Shapes {
@@ -1330,62 +952,11 @@ struct Shapes {
     int rr;               // rows per CTA in the inverse row pass (0: sequential kernel)
     int icols_cb;         // columns per CTA of the CTA-wide inverse column pass (0: warp kernel)
     int seq_sb;           // scales per engine call of the sequential row kernel
-    int row_eng, col_eng; // transform engine of the row / column length (engine_id)
     size_t sm_rows, sm_fcols, sm_icols, sm_irows, sm_icols_seq;
 };
 
-// Compiled transform engine serving a length: 1 (270) or 2 (480) when the length's own plan is
-// exactly the compiled radix sequence, else 0 (the runtime-planned engine).
-int engine_id(const iqm::FftLen &L) {
-    auto is = [&](int n, std::initializer_list<int> rs) {
-        if (L.bluestein || L.n != n || L.nst != int(rs.size())) return false;
-        int i = 0;
-        for (int r : rs)
-            if (L.radix[i++] != r) return false;
-        return true;
-    };
-    if (is(270, {9, 3, 10})) return 1;
-    if (is(480, {15, 8, 4})) return 2;
-    return 0;
-}
-
-// Work buffers per warp of engine `id` (matches engine_bufs of the types with_engine selects).
-int engine_buffers(int id) { return id == 2 ? 1 : 2; }
-static_assert(engine_bufs<Engine270>::value == 2 && engine_bufs<Engine480>::value == 1 &&
-                  engine_bufs<GenericEngine>::value == 2,
-              "engine_buffers() must match the engines' work buffers");
-
-template <class F>
-void with_engine(int id, F &&f) {
-    switch (id) {
-        case 1: f(Engine270{}); break;
-        case 2: f(Engine480{}); break;
-        default: f(GenericEngine{}); break;
-    }
-}
-
-// Warps of a kernel resident per SM at this block size and dynamic shared memory (raises the
-// kernel's shared-memory limit first, as a launch would).  Memoised per device: plane shapes are
-// chosen on every enqueue.
-int resident_warps(const void *fn, int threads, size_t smem) {
-    static std::mutex mu;
-    static std::map<std::tuple<int, const void *, int, size_t>, int> known;
-    int dev = 0;
-    IQM_CHECK_CUDA(cudaGetDevice(&dev));
-    const auto key = std::make_tuple(dev, fn, threads, smem);
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        auto it = known.find(key);
-        if (it != known.end()) return it->second;
-    }
-    set_smem(fn, smem);
-    int blocks = 0;
-    IQM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, threads, smem));
-    const int warps = blocks * threads / 32;
-    std::lock_guard<std::mutex> lock(mu);
-    known[key] = warps;
-    return warps;
-}
+// Warps of a kernel resident per SM at this block size and dynamic shared memory.
+int resident_warps(const void *fn, int threads, size_t smem) { return iqm::resident_ctas(fn, threads, smem) * threads / 32; }
 
 int lw_fit(size_t fixed, size_t per_warp) {
     int lw = 3;  // up to 8 warps
@@ -1398,24 +969,21 @@ Shapes shapes_for(const iqm::FsimPlan &P, const iqm::FsimTune &tune = iqm::FsimT
     const size_t f2 = sizeof(float2);
     s.wl_row = iqm::fft_work_len(P.row);
     s.wl_col = iqm::fft_work_len(P.col);
-    s.row_eng = engine_id(P.row);
-    s.col_eng = engine_id(P.col);
     const size_t twr = size_t((iqm::stage_twiddle_len(P.row) + 1) & ~1) * f2;
     const size_t twc = size_t((iqm::stage_twiddle_len(P.col) + 1) & ~1) * f2;
-    const size_t warp_row = engine_buffers(s.row_eng) * NB * size_t(s.wl_row) * f2;
-    const size_t warp_col = engine_buffers(s.col_eng) * NB * size_t(s.wl_col) * f2;
+    const size_t warp_row = 2 * NB * size_t(s.wl_row) * f2;
+    const size_t warp_col = 2 * NB * size_t(s.wl_col) * f2;
     s.lw_rows = lw_fit(twr, warp_row);
     s.sm_rows = twr + (size_t(1) << s.lw_rows) * warp_row;
     s.lw_fcols = lw_fit(twc, warp_col);
     s.sm_fcols = twc + (size_t(1) << s.lw_fcols) * warp_col;
     s.lw_icols = lw_fit(twc, warp_col + NB * size_t(P.h2) * f2);
-    if (tune.icols_lw >= 0) s.lw_icols = std::min(s.lw_icols, tune.icols_lw);
     s.sm_icols = twc + (size_t(1) << s.lw_icols) * (warp_col + NB * size_t(P.h2) * f2);
     // Runtime-planned columns: the CTA-wide column kernel (cb columns per CTA, the most warps resident
     // per SM) when it keeps at least twice as many warps resident as the warp kernel, whose per-warp
     // work buffers grow with the length.
-    if (s.col_eng == 0) {
-        const int w_warp = resident_warps((const void *)fsim_inv_cols_kernel<GenericEngine>, 32 << s.lw_icols, s.sm_icols);
+    {
+        const int w_warp = resident_warps((const void *)fsim_inv_cols_kernel, 32 << s.lw_icols, s.sm_icols);
         int best = 0;
         for (int cb : {4, 2, 1}) {
             const size_t sm = size_t(cb) * (size_t(P.h2) + 2 * size_t(s.wl_col)) * f2;
@@ -1459,16 +1027,10 @@ Shapes shapes_for(const iqm::FsimPlan &P, const iqm::FsimTune &tune = iqm::FsimT
 }
 
 void configure_kernels(const Shapes &s) {
-    with_engine(s.row_eng, [&](auto e) {
-        using E = decltype(e);
-        set_smem((const void *)fsim_fwd_rows_kernel<E>, s.sm_rows);
-        if (s.rr) set_smem((const void *)fsim_inv_rows_kernel<E>, s.sm_irows);
-    });
-    with_engine(s.col_eng, [&](auto e) {
-        using E = decltype(e);
-        set_smem((const void *)fsim_fwd_cols_kernel<E>, s.sm_fcols);
-        set_smem((const void *)fsim_inv_cols_kernel<E>, s.sm_icols);
-    });
+    set_smem((const void *)fsim_fwd_rows_kernel, s.sm_rows);
+    if (s.rr) set_smem((const void *)fsim_inv_rows_kernel, s.sm_irows);
+    set_smem((const void *)fsim_fwd_cols_kernel, s.sm_fcols);
+    set_smem((const void *)fsim_inv_cols_kernel, s.sm_icols);
     if (!s.rr) {
         set_smem((const void *)fsim_inv_rows_seq_kernel, s.sm_irows);
     }
@@ -1478,17 +1040,12 @@ void configure_kernels(const Shapes &s) {
 void launch_inv_rows(const FsimGroup &g, const iqm::FsimPlan &P, const Shapes &s, int planes, int consts_mode,
                      double *rowsums, cudaStream_t st) {
     if (s.rr && !(consts_mode && s.rr != 1)) {
-        with_engine(s.row_eng, [&](auto e) {
-            fsim_inv_rows_kernel<decltype(e)>
-                <<<dim3(iqm::ceil_div(P.h2, s.rr), 4, planes), 32 * (4 / NB) * s.rr, s.sm_irows, st>>>(
-                    g, P.row, s.wl_row, s.rr, consts_mode, rowsums);
-        });
+        fsim_inv_rows_kernel<<<dim3(iqm::ceil_div(P.h2, s.rr), 4, planes), 32 * (4 / NB) * s.rr, s.sm_irows, st>>>(
+            g, P.row, s.wl_row, s.rr, consts_mode, rowsums);
     } else if (s.rr) {  // consts mode runs one row per CTA
         const size_t twr = size_t((iqm::stage_twiddle_len(P.row) + 1) & ~1) * sizeof(float2);
-        with_engine(s.row_eng, [&](auto e) {
-            fsim_inv_rows_kernel<decltype(e)><<<dim3(P.h2, 4, planes), 32 * (4 / NB), twr + (s.sm_irows - twr) / s.rr, st>>>(
-                g, P.row, s.wl_row, 1, 1, rowsums);
-        });
+        fsim_inv_rows_kernel<<<dim3(P.h2, 4, planes), 32 * (4 / NB), twr + (s.sm_irows - twr) / s.rr, st>>>(
+            g, P.row, s.wl_row, 1, 1, rowsums);
     } else {
         fsim_inv_rows_seq_kernel<<<dim3(P.h2, 4, planes), FT, s.sm_irows, st>>>(g, P.row, s.wl_row, s.seq_sb,
                                                                                  consts_mode, rowsums);
@@ -1503,10 +1060,14 @@ void launch_inv_cols(const FsimGroup &g, const iqm::FsimPlan &P, const Shapes &s
         return;
     }
     const int nw = 1 << s.lw_icols;
-    with_engine(s.col_eng, [&](auto e) {
-        fsim_inv_cols_kernel<decltype(e)><<<dim3(iqm::ceil_div(P.w2, NB * nw), 4, planes), 32 * nw, s.sm_icols, st>>>(
-            g, P.col, s.wl_col, s.lw_icols, consts_mode);
-    });
+    fsim_inv_cols_kernel<<<dim3(iqm::ceil_div(P.w2, NB * nw), 4, planes), 32 * nw, s.sm_icols, st>>>(
+        g, P.col, s.wl_col, s.lw_icols, consts_mode);
+}
+
+// A spectrum of ones, whose filtered inverse transforms are those of the filters themselves.
+__global__ void fsim_ones_kernel(float2 *s, int n) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < n) s[p] = make_float2(1.f, 0.f);
 }
 
 iqm::FsimPlan *get_plan(iqm_ctx *ctx, int w2, int h2) {
@@ -1520,21 +1081,28 @@ iqm::FsimPlan *get_plan(iqm_ctx *ctx, int w2, int h2) {
     const int n = P->n;
     void *tmp = nullptr;
     try {
-        P->row = iqm::fft_len(ctx, w2);
-        P->col = iqm::fft_len(ctx, h2);
-        IQM_CHECK_CUDA(cudaMalloc(&P->filters, sizeof(float) * 16 * size_t(n)));
+        const iqm::RegFft *row = iqm::reg_fft_len(ctx, w2, P->krow), *col = iqm::reg_fft_len(ctx, h2, P->kcol);
+        P->reg = row && col;
+        if (P->reg) {
+            P->rrow = *row;
+            P->rcol = *col;
+            iqm::reg_tiles(*P);
+        } else {
+            P->row = iqm::fft_len(ctx, w2);
+            P->col = iqm::fft_len(ctx, h2);
+        }
+        const int planes_n = P->reg ? P->tiled : n;  // elements of a filter or spectrum plane
+        IQM_CHECK_CUDA(cudaMalloc(&P->filters, sizeof(float) * 16 * size_t(planes_n)));
         IQM_CHECK_CUDA(cudaMalloc(&P->consts, sizeof(double) * 20));
-        const Shapes s = shapes_for(*P);
-        configure_kernels(s);
         cudaStream_t st = ctx->stream;
-        fsim_filters_kernel<<<iqm::ceil_div(n, FT), FT, 0, st>>>(P->filters, w2, h2);
+        fsim_filters_kernel<<<iqm::ceil_div(n, FT), FT, 0, st>>>(P->filters, w2, h2, P->lc, P->tile, P->tiled);
         IQM_CHECK_CUDA(cudaGetLastError());
-        fsim_em_kernel<<<4, FT, 0, st>>>(P->filters, n, P->consts);
+        fsim_em_kernel<<<4, FT, 0, st>>>(P->filters, w2, h2, P->lc, P->tile, P->tiled, P->consts);
         IQM_CHECK_CUDA(cudaGetLastError());
         // transforms of the filters themselves
         const size_t tbytes = sizeof(float2) * 16 * size_t(n);
         const size_t rbytes = sizeof(double) * 4 * 4 * size_t(h2);
-        IQM_CHECK_CUDA(cudaMalloc(&tmp, tbytes + rbytes));
+        IQM_CHECK_CUDA(cudaMalloc(&tmp, tbytes + rbytes + sizeof(float2) * size_t(planes_n)));
         FsimGroup g{};
         g.G = 1;
         g.w2 = w2;
@@ -1543,9 +1111,24 @@ iqm::FsimPlan *get_plan(iqm_ctx *ctx, int w2, int h2) {
         g.T = static_cast<float2 *>(tmp);
         g.filters = P->filters;
         double *rowsums = reinterpret_cast<double *>(static_cast<uint8_t *>(tmp) + tbytes);
-        launch_inv_cols(g, *P, s, 1, 1, st);
-        IQM_CHECK_CUDA(cudaGetLastError());
-        launch_inv_rows(g, *P, s, 1, 1, rowsums, st);
+        if (P->reg) {
+            const iqm::RegShapes s = iqm::reg_shapes(*P, iqm::FsimTune{});
+            g.spec2 = reinterpret_cast<float2 *>(static_cast<uint8_t *>(tmp) + tbytes + rbytes);
+            g.lc = P->lc;
+            g.tile = P->tile;
+            g.tiled = P->tiled;
+            fsim_ones_kernel<<<iqm::ceil_div(P->tiled, FT), FT, 0, st>>>(g.spec2, P->tiled);
+            IQM_CHECK_CUDA(cudaGetLastError());
+            launch_reg_inv_cols(g, *P, s, 1, st);
+            IQM_CHECK_CUDA(cudaGetLastError());
+            launch_reg_inv_rows(g, *P, s, 1, rowsums, st);
+        } else {
+            const Shapes s = shapes_for(*P);
+            configure_kernels(s);
+            launch_inv_cols(g, *P, s, 1, 1, st);
+            IQM_CHECK_CUDA(cudaGetLastError());
+            launch_inv_rows(g, *P, s, 1, 1, rowsums, st);
+        }
         IQM_CHECK_CUDA(cudaGetLastError());
         fsim_consts_reduce_kernel<<<1, 32, 0, st>>>(rowsums, h2, P->consts);
         IQM_CHECK_CUDA(cudaGetLastError());
@@ -1571,19 +1154,20 @@ iqm::FsimPlan *get_plan(iqm_ctx *ctx, int w2, int h2) {
 }
 
 struct Layout {
-    size_t yiq, spec, T, planes, thr, partials, counters, total;
+    size_t yiq, spec, spec2, T, planes, thr, partials, counters, total;
 };
 
 // G pairs of the group; chunk pairs' worth of inverse-pass intermediates.
 // nbuf: inverse-pass intermediate buffers (2 when consecutive chunks alternate between two streams).
-// tbytes: bytes per element of the intermediate planes (8: FP32 complex, 4: FP16 complex).
-Layout layout_for(int G, int chunk, int n, int tiles, int nbuf = 1, size_t tbytes = sizeof(float2)) {
+// tiled: elements of a spectrum plane of the register engine (0: not used).
+Layout layout_for(int G, int chunk, int n, int tiles, int nbuf, int tiled) {
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     Layout L{};
     size_t off = 0;
     L.yiq = off; off += al(sizeof(float) * size_t(G) * 6 * n);
     L.spec = off; off += al(sizeof(float2) * size_t(G) * n);
-    L.T = off; off += al(tbytes * size_t(nbuf) * chunk * 32 * n);
+    L.spec2 = off; off += al(sizeof(float2) * size_t(G) * 2 * tiled);
+    L.T = off; off += al(sizeof(float2) * size_t(nbuf) * chunk * 32 * n);
     L.planes = off; off += al(sizeof(float) * size_t(G) * 24 * n);
     L.thr = off; off += al(sizeof(float) * size_t(G) * 8);
     L.partials = off; off += al(sizeof(double) * size_t(G) * tiles * 3);
@@ -1592,73 +1176,14 @@ Layout layout_for(int G, int chunk, int n, int tiles, int nbuf = 1, size_t tbyte
     return L;
 }
 
-// Inverse-pass chunk: the 32 intermediate planes of `chunk` pairs stay within an L2 budget
-// (80 MB unless tuned).
-int chunk_pairs(const iqm::FsimTune &t, int G, int n, size_t tbytes = sizeof(float2)) {
-    const size_t budget = size_t(t.chunk_mb > 0 ? t.chunk_mb : 80) << 20;
-    return std::max(1, std::min(G, int(budget / (tbytes * 32 * size_t(n)))));
-}
-
-// Tensor-core transform engines of the mixed forms exist for 480 x 270 planes (1080p and 4K pairs
-// downscale to them); other plane sizes run the FP32 transforms in the mixed forms too.
-bool mma_plane(int w2, int h2) { return w2 == 480 && h2 == 270; }
-
-// CTAs of a persistent kernel: the items, or as many CTAs as fit on the device at once.
-int persistent_grid(const void *fn, int threads, size_t smem, int items) {
-    int dev = 0, sms = 0, per_sm = 0;
-    IQM_CHECK_CUDA(cudaGetDevice(&dev));
-    IQM_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    set_smem(fn, smem);
-    IQM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
-    return std::max(1, std::min(items, sms * std::max(1, per_sm)));
-}
-
-// Offsets of the four engines' constant tables in FsimPlan::mma_tables.
-struct MmaTableLayout {
-    size_t col1, col3, row1, row3, total;
-};
-MmaTableLayout mma_table_layout() {
-    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    MmaTableLayout L{};
-    L.col1 = 0;
-    L.col3 = L.col1 + al(MmaCol270<1>::table_bytes);
-    L.row1 = L.col3 + al(MmaCol270<3>::table_bytes);
-    L.row3 = L.row1 + al(MmaRow480<1>::table_bytes);
-    L.total = L.row3 + al(MmaRow480<3>::table_bytes);
-    return L;
-}
-
-// pairs: pairs in the chunk (each item of the column pass covers both images of a pair).
-template <int SPLIT>
-void launch_inv_mma(const FsimGroup &g, const iqm::FsimPlan &P, int pairs, cudaStream_t st, iqm_ctx *ctx) {
-    using C = MmaCol270<SPLIT>;
-    using R = MmaRow480<SPLIT>;
-    const MmaTableLayout TL = mma_table_layout();
-    const uint8_t *tables = static_cast<const uint8_t *>(P.mma_tables);
-    const int citems = int(iqm::ceil_div(g.w2, MCW)) * 4 * pairs;
-    const size_t csm = MmaColGeom<C>::smem;
-    const int cgrid = persistent_grid((const void *)fsim_inv_cols_mma_kernel<C>, 32 * MCW, csm, citems);
-    fsim_inv_cols_mma_kernel<C><<<cgrid, 32 * MCW, csm, st>>>(g, tables + (SPLIT == 1 ? TL.col1 : TL.col3), citems);
-    iqm::check_launch(ctx, "fsim_inv_cols_mma_kernel");
-    const int ritems = g.h2 * 4 * 2 * pairs;
-    const size_t rsm = MmaRowGeom<R>::smem;
-    const int rgrid = persistent_grid((const void *)fsim_inv_rows_mma_kernel<R>, 32 * MRW, rsm,
-                                      int(iqm::ceil_div(ritems, MRW)));
-    fsim_inv_rows_mma_kernel<R><<<rgrid, 32 * MRW, rsm, st>>>(g, tables + (SPLIT == 1 ? TL.row1 : TL.row3), ritems);
-    iqm::check_launch(ctx, "fsim_inv_rows_mma_kernel");
-}
-
-// The tensor-core engines' constant tables of a 480 x 270 plan, built once on the context stream.
-void ensure_mma_tables(iqm_ctx *ctx, iqm::FsimPlan *P) {
-    if (P->mma_tables) return;
-    const MmaTableLayout TL = mma_table_layout();
-    IQM_CHECK_CUDA(cudaMalloc(&P->mma_tables, TL.total));
-    uint8_t *t = static_cast<uint8_t *>(P->mma_tables);
-    mma_table_kernel<MmaCol270<1>><<<1, 32, 0, ctx->stream>>>(t + TL.col1);
-    mma_table_kernel<MmaCol270<3>><<<1, 32, 0, ctx->stream>>>(t + TL.col3);
-    mma_table_kernel<MmaRow480<1>><<<1, 32, 0, ctx->stream>>>(t + TL.row1);
-    mma_table_kernel<MmaRow480<3>><<<1, 32, 0, ctx->stream>>>(t + TL.row3);
-    IQM_CHECK_CUDA(cudaGetLastError());
+// Inverse-pass chunk: the 32 intermediate planes of `chunk` pairs stay within a budget (640 MB unless
+// tuned).  The L2 would hold two 1080p pairs' planes, but launches of a pair or two leave the SMs half
+// empty for most of their time, which costs more than sending the planes through HBM.  32 1080p pairs in
+// budgets of 80 / 160 / 320 / 640 / 1200 MB: 1095 / 1094 / 1050 / 1017 / 1009 us; 32 pairs of 512x512:
+// 520 / 526 / 497 / 495 / 495 us.
+int chunk_pairs(const iqm::FsimTune &t, int G, int n) {
+    const size_t budget = size_t(t.chunk_mb > 0 ? t.chunk_mb : 640) << 20;
+    return std::max(1, std::min(G, int(budget / (sizeof(float2) * 32 * size_t(n)))));
 }
 
 void launch_ingest(const FsimGroup &g, int F_uniform, int tiles, cudaStream_t st) {
@@ -1673,9 +1198,7 @@ void launch_ingest(const FsimGroup &g, int F_uniform, int tiles, cudaStream_t st
 }
 
 // Enqueue FSIM for device-resident pairs; scores[2*i], scores[2*i+1] = FSIM, FSIMc of pair i.
-// mma: 0 = FP32 transforms; 1 or 3 = tensor-core transforms with that many products per tile
-// (1: FP16 operands, 3: split-precision hi + lo operands) where the plane size has MMA engines.
-void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_mode, int mma, double *d_scores) {
+void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_mode, double *d_scores) {
     const int n_pairs = int(pairs.size());
     // group by plane size, keeping the caller's order inside each group
     std::map<std::pair<int, int>, std::vector<int>> groups;
@@ -1698,10 +1221,10 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
     // per-size tables first (building one waits for the context stream)
     struct GroupRun {
         int w2, h2, G, first, slot, F_uniform, chunk;
-        int mma;       // tensor-core inverse passes (0: FP32 engines), FP16 intermediate planes
         bool overlap;  // inverse-pass chunks alternate between two streams and two T buffers
         iqm::FsimPlan *P;
         Shapes s;
+        iqm::RegShapes rs;
         Layout L;
         double cost;
     };
@@ -1715,17 +1238,16 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
             r.G = int(kv.second.size());
             r.first = first;
             r.P = get_plan(ctx, r.w2, r.h2);
-            r.s = shapes_for(*r.P, ctx->fsim_tune);
             const int n = r.P->n;
-            r.mma = mma_plane(r.w2, r.h2) ? mma : 0;
-            if (r.mma) ensure_mma_tables(ctx, r.P);
-            const size_t tbytes = r.mma ? sizeof(__half2) : sizeof(float2);
-            r.chunk = chunk_pairs(ctx->fsim_tune, r.G, n, tbytes);
-            // More than one chunk: split the L2 budget over two buffers and let consecutive chunks run
+            if (r.P->reg) r.rs = iqm::reg_shapes(*r.P, ctx->fsim_tune);
+            else r.s = shapes_for(*r.P, ctx->fsim_tune);
+            r.chunk = chunk_pairs(ctx->fsim_tune, r.G, n);
+            // More than one chunk: split the budget over two buffers and let consecutive chunks run
             // on two streams, so one chunk's column pass fills the other's last partial wave.
             r.overlap = kOverlapChunks && !ctx->timing && r.G > r.chunk;
             if (r.overlap) r.chunk = std::max(1, r.chunk / kChunkStreams);
-            r.L = layout_for(r.G, r.chunk, n, int(iqm::ceil_div(n, FT)), r.overlap ? kChunkStreams : 1, tbytes);
+            r.L = layout_for(r.G, r.chunk, n, int(iqm::ceil_div(n, FT)), r.overlap ? kChunkStreams : 1,
+                             r.P->tiled);
             r.F_uniform = hd[kv.second[0]].F;
             for (int i : kv.second)
                 if (hd[i].F != r.F_uniform) r.F_uniform = 0;
@@ -1775,7 +1297,8 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
         const Shapes &s = r.s;
         cudaStream_t st = streams[r.slot];
         uint8_t *base = base0 + slot_off[r.slot];
-        configure_kernels(s);
+        const bool reg = P->reg;
+        if (!reg) configure_kernels(s);
         const int n = P->n;
         const int tiles = int(iqm::ceil_div(n, FT));
         const int chunk = r.chunk;
@@ -1789,6 +1312,10 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
         g.n = n;
         g.yiq = reinterpret_cast<float *>(base + Lc.yiq);
         g.spec = reinterpret_cast<float2 *>(base + Lc.spec);
+        g.spec2 = reinterpret_cast<float2 *>(base + Lc.spec2);
+        g.lc = P->lc;
+        g.tile = P->tile;
+        g.tiled = P->tiled;
         g.T = reinterpret_cast<float2 *>(base + Lc.T);
         g.amp = reinterpret_cast<float *>(base + Lc.planes);
         g.energy = g.amp + size_t(G) * 8 * n;
@@ -1805,18 +1332,19 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
         iqm::timing_mark(ctx, nullptr);
         launch_ingest(g, r.F_uniform, tiles, st);
         iqm::check_launch(ctx, "fsim_ingest_kernel");
-        with_engine(s.row_eng, [&](auto e) {
-            fsim_fwd_rows_kernel<decltype(e)>
-                <<<dim3(iqm::ceil_div(h2, NB << s.lw_rows), G), 32 << s.lw_rows, s.sm_rows, st>>>(g, P->row,
-                                                                                                    s.wl_row);
-        });
-        iqm::check_launch(ctx, "fsim_fwd_rows_kernel");
-        with_engine(s.col_eng, [&](auto e) {
-            fsim_fwd_cols_kernel<decltype(e)>
-                <<<dim3(iqm::ceil_div(w2, NB << s.lw_fcols), G), 32 << s.lw_fcols, s.sm_fcols, st>>>(
-                    g, P->col, s.wl_col, s.lw_fcols);
-        });
-        iqm::check_launch(ctx, "fsim_fwd_cols_kernel");
+        if (reg) {
+            launch_reg_fwd_rows(g, *P, r.rs, st);
+            iqm::check_launch(ctx, "fsim_fwd_rows_kernel");
+            launch_reg_fwd_cols(g, *P, r.rs, st);
+            iqm::check_launch(ctx, "fsim_fwd_cols_kernel");
+        } else {
+            fsim_fwd_rows_kernel<<<dim3(iqm::ceil_div(h2, NB << s.lw_rows), G), 32 << s.lw_rows, s.sm_rows, st>>>(
+                g, P->row, s.wl_row);
+            iqm::check_launch(ctx, "fsim_fwd_rows_kernel");
+            fsim_fwd_cols_kernel<<<dim3(iqm::ceil_div(w2, NB << s.lw_fcols), G), 32 << s.lw_fcols, s.sm_fcols, st>>>(
+                g, P->col, s.wl_col, s.lw_fcols);
+            iqm::check_launch(ctx, "fsim_fwd_cols_kernel");
+        }
         // chunk k runs on stream k mod N of this slot (0: the group's stream) with buffer k mod N
         const int nst = r.overlap ? kChunkStreams : 1;
         cudaStream_t cstream[8] = {st};
@@ -1834,16 +1362,14 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
             const int j = k % nst;
             cudaStream_t cs = cstream[j];
             const int cg = std::min(chunk, G - c0);
-            if (r.mma) {
-                gc.Th = reinterpret_cast<__half2 *>(g.T) + size_t(j) * chunk * 32 * n;
-                gc.T = nullptr;
-                if (r.mma == 3)
-                    launch_inv_mma<3>(gc, *P, cg, cs, ctx);
-                else
-                    launch_inv_mma<1>(gc, *P, cg, cs, ctx);
+            gc.T = g.T + size_t(j) * chunk * 32 * n;
+            if (reg) {
+                launch_reg_inv_cols(gc, *P, r.rs, 2 * cg, cs);
+                iqm::check_launch(ctx, "fsim_inv_cols_kernel");
+                launch_reg_inv_rows(gc, *P, r.rs, 2 * cg, nullptr, cs);
+                iqm::check_launch(ctx, "fsim_inv_rows_kernel");
                 continue;
             }
-            gc.T = g.T + size_t(j) * chunk * 32 * n;
             launch_inv_cols(gc, *P, s, 2 * cg, 0, cs);
             iqm::check_launch(ctx, "fsim_inv_cols_kernel");
             launch_inv_rows(gc, *P, s, 2 * cg, 0, nullptr, cs);
@@ -1882,9 +1408,6 @@ void check_fsim_args(const iqm_pair *pairs, int n, iqm_precision precision, int 
     }
 }
 
-// Products per tensor-core tile of the mixed forms (0: the FP32 form).
-int mma_terms(iqm_precision p) { return p == IQM_MIXED ? 3 : p == IQM_MIXED_FAST ? 1 : 0; }
-
 }  // namespace
 
 void iqm_release_fsim_plans(iqm_ctx *ctx) {
@@ -1899,7 +1422,7 @@ void iqm::enqueue_fsim_dev(iqm_ctx *ctx, const iqm_pair *pairs, int n, iqm_preci
     check_fsim_args(pairs, n, precision, energy_mode);
     iqm::check_dev_alignment(pairs, n);
     IQM_REQUIRE(d_scores != nullptr, "d_scores is NULL");
-    fsim_enqueue(ctx, std::vector<iqm_pair>(pairs, pairs + n), energy_mode, mma_terms(precision), d_scores);
+    fsim_enqueue(ctx, std::vector<iqm_pair>(pairs, pairs + n), energy_mode, d_scores);
 }
 
 IQM_API int iqm_fsim_dev(iqm_ctx *ctx, const iqm_pair *pairs, int n, iqm_precision precision, int energy_mode,
@@ -1914,8 +1437,7 @@ IQM_API int iqm_fsim_batch(iqm_ctx *ctx, const iqm_pair *pairs, int n, iqm_preci
         IQM_REQUIRE(scores != nullptr, "scores is NULL");
         auto *d_scores = static_cast<double *>(ctx->scores.get(sizeof(double) * 2 * n, ctx->stream));
         iqm::upload_pipelined(ctx, pairs, n, [&](const iqm_pair *dev, int first, int count) {
-            fsim_enqueue(ctx, std::vector<iqm_pair>(dev, dev + count), energy_mode, mma_terms(precision),
-                         d_scores + 2 * first);
+            fsim_enqueue(ctx, std::vector<iqm_pair>(dev, dev + count), energy_mode, d_scores + 2 * first);
         });
         IQM_CHECK_CUDA(cudaMemcpyAsync(scores, d_scores, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, ctx->stream));
         IQM_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1930,7 +1452,7 @@ IQM_API int iqm_fsim(iqm_ctx *ctx, const uint8_t *rgba_in, const uint8_t *rgba_r
         check_fsim_args(&hp, 1, precision, energy_mode);
         auto dev = iqm::upload_pairs(ctx, &hp, 1);
         auto *d_scores = static_cast<double *>(ctx->scores.get(sizeof(double) * 2, ctx->stream));
-        fsim_enqueue(ctx, dev, energy_mode, mma_terms(precision), d_scores);
+        fsim_enqueue(ctx, dev, energy_mode, d_scores);
         double out[2];
         IQM_CHECK_CUDA(cudaMemcpyAsync(out, d_scores, sizeof(out), cudaMemcpyDeviceToHost, ctx->stream));
         IQM_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));

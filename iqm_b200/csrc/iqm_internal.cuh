@@ -112,13 +112,13 @@ struct UploadRing {
 // Launch-shape choices of the FSIM transform passes (0 / -1 = built-in heuristic).  They change
 // only how work is split over CTAs, never a result bit; batch plans autotune them (plan.cu).
 struct FsimTune {
-    int chunk_mb = 0;     // L2 budget for the inverse-pass intermediates of one chunk of pairs
-    int icols_lw = -1;    // log2 warps per CTA of the inverse column pass (clamped to what fits)
+    int chunk_mb = 0;     // budget for the inverse-pass intermediates of one chunk of pairs
     int rows_per_cta = 0; // rows per CTA of the inverse row pass (1 or 2, if it fits)
 };
 
 struct FsimPlan;  // per plane-size FSIM constants (fsim.cu)
 struct FftPlan;   // per-length FFT tables (fft.cu)
+struct RegPlan;   // per-length plans of the register FFT engine (fft_reg.cu)
 
 }  // namespace iqm
 
@@ -151,6 +151,7 @@ struct iqm_ctx {
 
     std::map<std::pair<int, int>, iqm::FsimPlan *> fsim_plans;  // owned; freed by iqm_release_fsim_plans
     std::map<int, iqm::FftPlan *> fft_plans;  // owned; freed by iqm_release_fft_plans
+    std::map<int, iqm::RegPlan *> reg_plans;  // owned; freed by iqm_release_reg_plans
 
     // Per-kernel device timing (iqm_set_kernel_timing): an event after every launch and after every
     // copy or memset the context enqueues; a kernel is charged the interval since the event before it.
@@ -278,6 +279,11 @@ __device__ __forceinline__ float rsqrt_approx(float x) {  // 1 / sqrt(x)
 __device__ __forceinline__ float rcp_approx(float x) {  // 1 / x
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {  // sqrt(x), x >= 0
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 // sqrt(v) for v >= 0 as v * rsqrt(v); 0 for v = 0

@@ -131,8 +131,8 @@ struct iqm_batch_plan {
         return ms / 2.f;
     }
 
-    // Coordinate search over the FSIM shapes: L2 budget of an inverse-pass chunk, warps per CTA of
-    // the inverse column pass, rows per CTA of the inverse row pass.  A candidate must be 2% faster
+    // Coordinate search over the FSIM shapes: budget of an inverse-pass chunk, rows per CTA of
+    // the inverse row pass.  A candidate must be 2% faster
     // to replace the current choice.
     void autotune_fsim() {
         cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -148,15 +148,9 @@ struct iqm_batch_plan {
                     best = t;
                 }
             };
-            for (int mb : {40, 160}) {
+            for (int mb : {80, 1280}) {
                 iqm::FsimTune t = best;
                 t.chunk_mb = mb;
-                consider(t);
-            }
-            const iqm::FsimTune base = best;
-            for (int lw : {2, 1}) {
-                iqm::FsimTune t = base;
-                t.icols_lw = lw;
                 consider(t);
             }
             {
@@ -166,8 +160,8 @@ struct iqm_batch_plan {
             }
             tune = best;
             char line[160];
-            std::snprintf(line, sizeof(line), "fsim: chunk_mb=%d icols_lw=%d rows_per_cta=%d (%.3f ms per batch)",
-                          tune.chunk_mb ? tune.chunk_mb : 80, tune.icols_lw, tune.rows_per_cta, double(best_ms));
+            std::snprintf(line, sizeof(line), "fsim: chunk_mb=%d rows_per_cta=%d (%.3f ms per batch)",
+                          tune.chunk_mb ? tune.chunk_mb : 640, tune.rows_per_cta, double(best_ms));
             info += line;
         } catch (...) {
             cudaEventDestroy(e0);

@@ -40,7 +40,7 @@
 // as the tensor cores see it (FP16-rounded taps in the fast form).
 #pragma once
 
-#include "dft_mma.cuh"
+#include "mma_f16.cuh"
 
 namespace {
 
