@@ -9,10 +9,9 @@
 // Here everything runs on the device in two kernels:
 //   msvd_block_kernel  two lanes per block slot (one per image): 8 rows x 8 RGBA8 pixels straight
 //                      into registers (two 16-byte loads per row, coalesced across a warp of
-//                      horizontally adjacent blocks), OpenCV's 15-bit fixed-point grey, one-sided
-//                      Jacobi SVD in registers (FP32 rotations, inner products and rotation test,
-//                      two rows per packed FP32x2 instruction; FP64 final norms), D in FP32 as the
-//                      shader does;
+//                      horizontally adjacent blocks), OpenCV's 15-bit fixed-point grey, singular
+//                      values in registers by bidiagonalisation (two rows per packed FP32x2
+//                      instruction) and differential qd sweeps, D in FP32 as the shader does;
 //   msvd_pool_kernel   one CTA per pair: exact median by radix select (select.cuh), then the mean
 //                      absolute deviation summed in FP64, and the optional D/max(D) map.
 #include <cfloat>
@@ -47,10 +46,13 @@ struct MsvdArgs {
     double *scores;      // npairs
 };
 
-__device__ __forceinline__ float gray_u8(uint32_t px) {
-    // cv::cvtColor(COLOR_RGB2GRAY) on 8-bit data: (R*9798 + G*19235 + B*3735 + 2^14) >> 15
-    const uint32_t r = px & 0xffu, g = (px >> 8) & 0xffu, b = (px >> 16) & 0xffu;
-    return float((r * 9798u + g * 19235u + b * 3735u + 16384u) >> 15);
+// cv::cvtColor(COLOR_RGB2GRAY) on 8-bit data: (R*9798 + G*19235 + B*3735 + 2^14) >> 15, in [0, 255], as
+// 2^23 + value: the weighted sum is two 16-by-8-bit dot products (the alpha byte weighs 0), and the
+// funnel shift that drops its 15 low bits brings the exponent of 2^23 in from above.
+__device__ __forceinline__ float gray_plus_2p23(uint32_t px) {
+    unsigned s = __dp2a_lo(9798u | 19235u << 16, px, 16384u);
+    s = __dp2a_hi(3735u, px, s);
+    return __uint_as_float(__funnelshift_r(s, 0x4B000000u >> 17, 15));
 }
 
 __device__ __forceinline__ int find_pair(const MsvdPairDev *p, int n, int slot) {
@@ -80,85 +82,193 @@ __device__ __forceinline__ void load_block(const uint8_t *img, long long pitch, 
         }
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-            if (r & 1) c[q][r >> 1].y = gray_u8(px[q]);
-            else c[q][r >> 1].x = gray_u8(px[q]);
+            if (r & 1) c[q][r >> 1].y = gray_plus_2p23(px[q]);
+            else c[q][r >> 1].x = gray_plus_2p23(px[q]);
         }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) c[q][k] = iqm::add2(c[q][k], iqm::dup2(-8388608.0f));
+}
+
+// sqrt(x) and 1 / x for normal x > 0 to within an ulp: one Newton step on the SFU's values
+__device__ __forceinline__ float sqrt_newton(float x) {
+    const float r = iqm::rsqrt_approx(x), y = x * r;
+    return fmaf(0.5f * r, fmaf(-y, y, x), y);
+}
+__device__ __forceinline__ float rcp_newton(float x) {
+    const float y = iqm::rcp_approx(x);
+    return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
+
+// A Householder reflection I - beta v v' that takes a vector of squared norm nn and first element x0 to
+// (alpha, 0, ...): v is the vector with x0 - alpha in place of x0.  A vector of zeros is left as it is
+// (beta 0), which also covers vectors of rounding noise too small for the squares of FP32.
+__device__ __forceinline__ void reflection(float nn, float x0, float &alpha, float &beta) {
+    const bool live = nn > 1e-30f;
+    const float norm = sqrt_newton(fmaxf(nn, 1e-30f));
+    alpha = live ? -copysignf(norm, x0) : 0.0f;
+    beta = live ? rcp_newton(fmaf(fabsf(x0), norm, nn)) : 0.0f;
+}
+
+// Step K of the bidiagonalisation: column K is reflected to its diagonal element d, then row K right of
+// it to e (the next two columns' element).  Rows go two to a register pair; rows above K in a pair that
+// straddles it are dead and may take any value.
+template <int K>
+__device__ __forceinline__ void bidiagonal_step(float2 (&c)[8][4], float (&d)[8], float (&e)[7]) {
+    if constexpr (K < 7) {
+        constexpr int P0 = K >> 1;  // first pair with rows >= K
+        float2 v[4];
+#pragma unroll
+        for (int p = P0; p < 4; p++) v[p] = c[K][p];
+        if (K & 1) v[P0].x = 0.f;
+        float2 n2 = iqm::mul2(v[P0], v[P0]);
+#pragma unroll
+        for (int p = P0 + 1; p < 4; p++) n2 = iqm::fma2(v[p], v[p], n2);
+        float beta;
+        const float x0 = (K & 1) ? v[P0].y : v[P0].x;
+        reflection(n2.x + n2.y, x0, d[K], beta);
+        if (K & 1) v[P0].y = x0 - d[K];
+        else v[P0].x = x0 - d[K];
+#pragma unroll
+        for (int j = K + 1; j < 8; j++) {
+            float2 s2 = iqm::mul2(v[P0], c[j][P0]);
+#pragma unroll
+            for (int p = P0 + 1; p < 4; p++) s2 = iqm::fma2(v[p], c[j][p], s2);
+            const float2 s = iqm::dup2(-beta * (s2.x + s2.y));
+#pragma unroll
+            for (int p = P0; p < 4; p++) c[j][p] = iqm::fma2(s, v[p], c[j][p]);
+        }
+    } else {
+        d[7] = c[7][3].y;
+    }
+    if constexpr (K < 6) {
+        constexpr int R = K >> 1, P0 = (K + 1) >> 1;  // row K's pair, first pair with rows > K
+        float v[8];
+        float nn = 0.f;
+#pragma unroll
+        for (int j = K + 1; j < 8; j++) {
+            v[j] = (K & 1) ? c[j][R].y : c[j][R].x;
+            nn = fmaf(v[j], v[j], nn);
+        }
+        float beta;
+        reflection(nn, v[K + 1], e[K], beta);
+        v[K + 1] -= e[K];
+        float2 s[4];
+#pragma unroll
+        for (int j = K + 1; j < 8; j++)
+#pragma unroll
+            for (int p = P0; p < 4; p++)
+                s[p] = j == K + 1 ? iqm::mul2(iqm::dup2(v[j]), c[j][p]) : iqm::fma2(iqm::dup2(v[j]), c[j][p], s[p]);
+#pragma unroll
+        for (int p = P0; p < 4; p++) s[p] = iqm::mul2(s[p], iqm::dup2(-beta));
+#pragma unroll
+        for (int j = K + 1; j < 8; j++)
+#pragma unroll
+            for (int p = P0; p < 4; p++) c[j][p] = iqm::fma2(iqm::dup2(v[j]), s[p], c[j][p]);
+    } else if constexpr (K == 6) {
+        e[6] = c[7][3].x;
     }
 }
 
-// <ci, cj> over the 8 rows: the even and odd rows as the two halves of packed FMAs, then their sum
-__device__ __forceinline__ float dot8(const float2 (&ci)[4], const float2 (&cj)[4]) {
-    float2 q = iqm::mul2(ci[0], cj[0]);
+// State of the quotient-difference iteration on the squares q of the diagonal and e of the superdiagonal.
+struct QdState {
+    float q[8], e[7];
+    float sigma;   // shifts applied so far: an eigenvalue is sigma + its q
+    float s1, s2;  // sums of 1 / x and 1 / x^2 over the eigenvalues of all rows but the last swept one
+};
+
+// Laguerre's lower bound of the smallest of m positive numbers whose reciprocals and their squares sum to
+// s1 and s2, a little less; 0 where the sums are not usable.
+__device__ __forceinline__ float laguerre_shift(float m, float s1, float s2) {
+    const float root = iqm::sqrt_approx(fmaxf((m - 1.0f) * fmaf(m, s2, -s1 * s1), 0.0f));
+    const float t = 0.9999f * m * iqm::rcp_approx(s1 + root);
+    return t > 1e-6f ? t : 0.0f;  // below 1e-6 (a singular value of 1e-3) the plain iteration converges at once
+}
+
+// Finds the smallest eigenvalue of the leading M rows and leaves it in q[M - 1] + sigma: shifted
+// differential qd sweeps until the last superdiagonal element no longer moves a singular value by 1e-5.
+// Every sweep also carries the first two derivatives of its pivots by the shift, which give the sums over
+// 1 / x and 1 / x^2 of the swept matrix's eigenvalues and with them the next shift; the sums without the
+// last pivot are those of the matrix that is left when the last row splits off.
+template <int M>
+__device__ __forceinline__ void qd_smallest(QdState &z) {
+    constexpr float kTiny = 1e-10f;
+    float tau = M == 8 ? 0.0f : laguerre_shift(float(M), z.s1, z.s2);
+#pragma unroll 1
+    for (int it = 0; it < 24; it++) {
+        const float el = z.e[M - 2];
+        if (el * el <= fmaxf(1e-10f * (z.sigma + z.q[M - 1]), 1e-18f)) break;
+        float Q[M], E[M - 1];
+        float dd = z.q[0] - tau, low = dd, d1 = -1.0f, d2 = 0.0f, s1 = 0.0f, s2 = 0.0f;
 #pragma unroll
-    for (int k = 1; k < 4; k++) q = iqm::fma2(ci[k], cj[k], q);
-    return q.x + q.y;
+        for (int i = 0; i < M - 1; i++) {
+            Q[i] = dd + z.e[i];
+            const float r = iqm::rcp_approx(fmaxf(Q[i], kTiny));
+            const float t = z.q[i + 1] * r;
+            E[i] = z.e[i] * t;
+            const float a = d1 * r, w = E[i] * r;
+            s1 -= a;
+            s2 = fmaf(-d2, r, fmaf(a, a, s2));
+            d2 = w * fmaf(-2.0f * a, d1, d2);
+            d1 = fmaf(w, d1, -1.0f);
+            dd = fmaf(dd, t, -tau);
+            low = fminf(low, dd);
+        }
+        Q[M - 1] = dd;
+        if (low >= 0.0f) {
+#pragma unroll
+            for (int i = 0; i < M; i++) z.q[i] = Q[i];
+#pragma unroll
+            for (int i = 0; i < M - 1; i++) z.e[i] = E[i];
+            z.sigma += tau;
+            z.s1 = s1;
+            z.s2 = s2;
+            const float r = iqm::rcp_approx(fmaxf(dd, kTiny)), a = d1 * r;
+            tau = laguerre_shift(float(M), s1 - a, fmaf(-d2, r, fmaf(a, a, s2)));
+        } else {
+            tau = 0.0f;  // the shift passed the smallest eigenvalue: sweep again without one
+        }
+    }
+    z.q[M - 1] += z.sigma;
 }
 
 // Singular values (descending) of the 8x8 matrix whose columns are c[0..7]; c is destroyed.
-// One-sided Jacobi: each (i, j) column pair is rotated so the columns become orthogonal.  Inner
-// products, rotations and the squared column norms (recomputed from the rotated columns) are FP32,
-// two rows per packed FP32x2 instruction (half the instructions and half the unrolled code of the
-// sweep, which otherwise overflows the instruction cache); the rotation test
-// |<ci,cj>|^2 > eps^2 |ci|^2 |cj|^2 is FP32 too (eps = 4 FLT_EPSILON, above FP32 rounding noise, so
-// sweeps stop: at most 6 on the OpenCV fixture blocks), and the final norms are accumulated in FP64
-// like OpenCV's Jacobi SVD.
-__device__ __forceinline__ void svd8_values(float2 c[8][4], float s[8]) {
-    float nrm[8];
+// Householder reflections to bidiagonal form, then the singular values of that by shifted differential
+// qd sweeps (K. V. Fernando and B. N. Parlett, "Accurate singular values and differential qd algorithms",
+// 1994), smallest first, with Laguerre's shifts.  On 8.1k blocks of an 8x8-quantised image the largest
+// deviation from double-precision singular values is 4.5e-4 and the RMS 3.9e-5 (values up to 2040); the
+// one-sided Jacobi method that this replaced had 6.3e-4 and 6.6e-5 and took about twice the time, six to
+// eight sweeps of 28 rotations.
+__device__ __forceinline__ void svd8_values(float2 (&c)[8][4], float s[8]) {
+    QdState z;
+    {
+        float d[8], e[7];
+        bidiagonal_step<0>(c, d, e);
+        bidiagonal_step<1>(c, d, e);
+        bidiagonal_step<2>(c, d, e);
+        bidiagonal_step<3>(c, d, e);
+        bidiagonal_step<4>(c, d, e);
+        bidiagonal_step<5>(c, d, e);
+        bidiagonal_step<6>(c, d, e);
+        bidiagonal_step<7>(c, d, e);
 #pragma unroll
-    for (int i = 0; i < 8; i++) nrm[i] = dot8(c[i], c[i]);
-    const float eps2 = 16.0f * FLT_EPSILON * FLT_EPSILON;
-    for (int sweep = 0; sweep < 60; sweep++) {
-        bool changed = false;
+        for (int i = 0; i < 8; i++) z.q[i] = d[i] * d[i];
 #pragma unroll
-        for (int i = 0; i < 7; i++) {
-#pragma unroll
-            for (int j = i + 1; j < 8; j++) {
-                const float p = dot8(c[i], c[j]);
-                // all three products stay far inside FP32's range (norms < 2^20); pairs whose inner
-                // product is below 1e-15 count as orthogonal, so columns that shrink to rounding
-                // noise do not keep the sweeps going through denormal products
-                if (p * p > fmaxf(eps2 * nrm[i] * nrm[j], 1e-30f)) {
-                    // 1e-15 < |p| <= |ci||cj| < 2^20 here, so the SFU reciprocal is accurate to a few
-                    // ulp; the angle only steers the sweep, later rotations remove what it leaves
-                    const float zeta = (nrm[j] - nrm[i]) * iqm::rcp_approx(2.0f * p);
-                    const float az = fabsf(zeta);
-                    // tan(theta): smaller root of t^2 + 2 zeta t - 1 = 0 (1/(2 zeta) once zeta^2
-                    // overflows); sqrt(z) as z rsqrt(z) for z = zeta^2 + 1 >= 1, and the SFU
-                    // reciprocal of a denominator in [1, 2^61)
-                    const float z = fmaf(zeta, zeta, 1.0f);
-                    const float t = copysignf(1.0f, zeta) * iqm::rcp_approx(az < 1e18f ? az + z * iqm::rsqrt_approx(z) : 2.0f * az);
-                    const float cs = iqm::rsqrt_approx(fmaf(t, t, 1.0f));
-                    const float sn = cs * t;
-                    const float2 cs2 = iqm::dup2(cs), sn2 = iqm::dup2(sn), msn2 = iqm::dup2(-sn);
-                    float2 ni = iqm::dup2(0.f), nj = iqm::dup2(0.f);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const float2 xi = c[i][k], xj = c[j][k];
-                        const float2 yi = iqm::fma2(cs2, xi, iqm::mul2(msn2, xj));
-                        const float2 yj = iqm::fma2(sn2, xi, iqm::mul2(cs2, xj));
-                        c[i][k] = yi;
-                        c[j][k] = yj;
-                        ni = iqm::fma2(yi, yi, ni);
-                        nj = iqm::fma2(yj, yj, nj);
-                    }
-                    nrm[i] = ni.x + ni.y;
-                    nrm[j] = nj.x + nj.y;
-                    changed = true;
-                }
-            }
-        }
-        if (!changed) break;
+        for (int i = 0; i < 7; i++) z.e[i] = e[i] * e[i];
     }
+    z.sigma = z.s1 = z.s2 = 0.0f;
+    qd_smallest<8>(z);
+    qd_smallest<7>(z);
+    qd_smallest<6>(z);
+    qd_smallest<5>(z);
+    qd_smallest<4>(z);
+    qd_smallest<3>(z);
+    qd_smallest<2>(z);
+    z.q[0] += z.sigma;
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        double q = 0.0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            q = fma(double(c[i][k].x), double(c[i][k].x), q);
-            q = fma(double(c[i][k].y), double(c[i][k].y), q);
-        }
-        s[i] = float(sqrt(q));
-    }
+    for (int i = 0; i < 8; i++) s[i] = z.q[i] > 1e-30f ? sqrt_newton(z.q[i]) : 0.0f;
     // descending order (sorting network on 8 registers)
 #define IQM_CSWAP(a, b)                         \
     do {                                        \
@@ -180,9 +290,10 @@ __device__ __forceinline__ void svd8_values(float2 c[8][4], float s[8]) {
 // Two lanes per block slot: the even lane takes the block of the distorted image, the odd lane the
 // same block of the reference; the odd lane's singular values reach the even lane by shuffle.  One
 // copy of the SVD code serves both images and twice as many blocks are in flight.
-// Five CTAs per SM (90 registers, no spills): with the packed row pairs, six CTAs at 80 registers
-// spill the columns and measured 16% slower.
-__global__ void __launch_bounds__(BLOCK_THREADS, 5) msvd_block_kernel(MsvdArgs args) {
+// Bound by instruction issue (72% of the issue slots, FMA pipe 52%, 4.7k instructions a block of one
+// image, about a sixth of them lost to lanes that wait for their warp's slowest qd sweep).  16 1080p
+// pairs: 475 us with Jacobi sweeps, 178 us now; five CTAs per SM at 93 registers 185 us, six at 80 178 us.
+__global__ void __launch_bounds__(BLOCK_THREADS, 6) msvd_block_kernel(MsvdArgs args) {
     const int slot = (blockIdx.x * BLOCK_THREADS + threadIdx.x) >> 1;
     const int img = threadIdx.x & 1;
     const bool in_range = slot < args.total_slots;  // both lanes of a slot agree
