@@ -43,13 +43,12 @@ extern "C" {
 
 typedef struct iqm_ctx iqm_ctx;
 
+/* Least precision that a caller accepts.  The FP32 kernels are now also the fastest of every metric, so
+ * all three values compute plain FP32 arithmetic with FP64 pooling sums. */
 typedef enum {
-    IQM_FP32 = 0,       /* plain FP32 arithmetic, FP64 pooling sums                              */
-    IQM_MIXED = 1,      /* SSIM: the Gaussian window sums on the tensor cores, moments staged as
-                           FP16 hi + lo pairs, split-precision products, FP32 accumulation.
-                           Scores within 1e-4 of the FP64 oracle.  FSIM, FLIP and M-SVD compute in
-                           FP32 whatever is asked.                                                 */
-    IQM_MIXED_FAST = 2  /* as IQM_MIXED with single FP16 operands and products (hi parts only)  */
+    IQM_FP32 = 0,
+    IQM_MIXED = 1,
+    IQM_MIXED_FAST = 2
 } iqm_precision;
 
 /* ---- context --------------------------------------------------------------------------- */
@@ -95,7 +94,7 @@ int iqm_ssim(iqm_ctx *ctx, const uint8_t *rgba_in, const uint8_t *rgba_ref, int 
  * contexts, or after cudaDeviceReset, are not supported.  All calls share the one array: calls
  * that overlap on the GPU (other streams, other threads) race -- serialise them.  `d_in`, `d_ref`,
  * `row_bytes` and `d_map` must be multiples of 4 and `d_mssim` of 8 (else IQM_EINVAL, before any
- * launch).  Only IQM_FP32 is served here: another `params->precision` returns IQM_EINVAL.
+ * launch).  Only IQM_FP32 is taken here: another `params->precision` returns IQM_EINVAL.
  * Returns IQM_OK, IQM_EINVAL (null or misaligned pointer, size or parameter out of range) or IQM_ECUDA (a launch of this call failed; errors pending from the caller's earlier work
  * are left pending, not reported or cleared). */
 #define IQM_SSIM_NOALLOC_MAX_TILES 4096

@@ -25,8 +25,9 @@ IQM_ENOMEM = -3
 IQM_EUNSUPPORTED = -4
 
 IQM_FP32 = 0
-IQM_MIXED = 1       # SSIM's window sums on the tensor cores, split-precision (hi + lo) FP16 products
-IQM_MIXED_FAST = 2  # the same with single FP16 products
+# least precision that the caller accepts; every metric computes FP32 whichever is given
+IQM_MIXED = 1
+IQM_MIXED_FAST = 2
 
 # every symbol include/iqm_cuda.h declares
 EXPORTS = (
@@ -263,7 +264,7 @@ class SSIM:
         self.k_1 = 0.01
         self.k_2 = 0.03
         self.sigma = 1.5
-        self.precision = IQM_FP32  # IQM_MIXED / IQM_MIXED_FAST: tensor-core window sums
+        self.precision = IQM_FP32
 
     def params(self):
         return SSIMParams(self.kernel_size, self.k_1, self.k_2, self.sigma, self.precision)

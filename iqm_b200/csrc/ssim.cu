@@ -15,14 +15,17 @@
 //     cov_ab = (var_u - var_v)/4, var_a + var_b = (var_u + var_v)/2;
 //   * the second moments are taken about a per-tile constant (the u, v of the tile's centre
 //     pixel), var = E[(x-c)^2] - E[x-c]^2, which keeps FP32 cancellation ~1e-7 on MSSIM;
-//   * each CTA owns a 128-column strip of ~120 output rows and streams down it: raw RGBA8 rows
-//     (plus a 5-pixel halo) are prefetched PF rows ahead with cp.async into a small shared ring,
-//     converted once to shifted (u, v), filtered horizontally from shared memory and pushed into a
-//     register ring of 2R+1 rows that carries the vertical taps (one barrier per row, ~11 KB of
-//     shared memory per CTA, so many CTAs overlap their loads with arithmetic);
+//   * lumas stay whole numbers, 299 R + 581 G + 114 B, so (u, v) and their distance to the constant are
+//     exact in FP32 until the first tap multiplies them;
+//   * each CTA owns a 128-column strip and streams down it four rows a step: the rows' (u, v) go to
+//     shared memory, a warp a row filters them horizontally, four neighbouring columns a lane (a
+//     staged value is loaded and squared once for the eleven outputs it serves), and a thread a column
+//     runs the vertical taps as a transposed filter, whose running sums move up one register a row, so
+//     that the row loop needs no unrolling over the window;
 //   * (u, v) pairs are processed with packed FP32x2 instructions (__ffma2_rn and friends);
-//   * MSSIM partials go to per-tile FP64 slots; the last CTA of a pair sums them in a fixed order
-//     (deterministic, no second launch).
+//   * MSSIM pools four rows of a column in FP32 and those sums in fixed point: neither the sum
+//     nor any per-pixel value depends on how an image is cut into strips, which is chosen per launch
+//     (strip_rows) from the number of images in it; the last CTA of a pair writes its mean.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -33,23 +36,22 @@
 namespace {
 
 constexpr int TW = 128;             // output columns per CTA (one vertical strip)
-constexpr int NT = TW;              // threads per CTA, one output column each
-constexpr int SMEM_COLS = TW + 16;  // staged columns x0-8 .. x0+TW+7 (16-byte aligned start)
-constexpr int NRAW = 8;             // raw RGBA row ring
-constexpr int PF = 6;               // rows prefetched ahead (< NRAW)
-
-template <int R>
-struct Geom {
-    static constexpr int K = 2 * R + 1;
-    // strip height: S + 2R is a multiple of K so the register ring indexes statically
-    static constexpr int S = K * ((120 + 2 * R + K - 1) / K) - 2 * R;
-    static constexpr int ROWS = S + 2 * R;
-};
+constexpr int NT = TW;              // threads per CTA: a vertical column each
+constexpr int RSTEP = 4;            // rows per step: a warp each in the horizontal pass
+constexpr int UNITS = (TW + 16) / 2;  // staged columns x0-8 .. x0+TW+7 of a row, two to a 16-byte unit
+constexpr int CHUNKS = (TW + 16) / 4; // 4-pixel loads of a row
+constexpr int SHIFT_ROWS = 128;     // rows that share a shift constant; strips divide it
+constexpr float LUMA_UNIT = 255000.0f;  // a luma of 1 in the whole numbers used here
 
 struct Smem {
-    uint32_t raw[NRAW][2][SMEM_COLS];  // RGBA8 rows of both images, as loaded
-    float2 uv[2][SMEM_COLS];           // shifted (u, v) of the row being filtered
+    float4 uv[RSTEP][UNITS];  // shifted (u, v) of two columns, at unit_at(flat index)
+    float4 h[RSTEP][TW];      // horizontal sums (g u, g v, g u^2, g v^2), at column_at(column)
 };
+
+// Neighbouring lanes of the horizontal pass read every other unit and write every fourth column; these
+// permutations spread them over the banks.
+__device__ __forceinline__ int unit_at(int p) { return p ^ ((p >> 3) & 1); }
+__device__ __forceinline__ int column_at(int c) { return c ^ ((c >> 3) & 3); }
 
 struct SsimPairDev {
     const uint8_t *a;
@@ -61,7 +63,6 @@ struct SsimPairDev {
     int tile_base;     // first global tile index of this pair
     int ntiles;
     int vec_ok;        // 16-byte loads allowed
-    int unit_base;     // tensor-core kernel: first global work unit (column segment of tiles)
 };
 
 struct SsimArgs {
@@ -70,17 +71,21 @@ struct SsimArgs {
     double *partials;    // one per tile
     unsigned *counters;  // one per pair, zero on entry
     double *scores;      // one per pair
-    float g[15];         // 1-D Gaussian taps g(-R..R)
-    float c1, c2;
+    int strip;           // rows of a tile
+    float2 g[8];         // 1-D Gaussian taps g(0..R), in both halves
+    float c1, c2;        // in squared luma units
 };
 
-// shaders/ssim/ssim_lumapack.glsl:19-21 (G weight 0.581 as in the reference) on unorm bytes
-__device__ __forceinline__ float luma_u8(uint32_t px) {
-    float r = float(px & 0xffu) * (1.0f / 255.0f);
-    float g = float((px >> 8) & 0xffu) * (1.0f / 255.0f);
-    float b = float((px >> 16) & 0xffu) * (1.0f / 255.0f);
-    return 0.299f * r + 0.581f * g + 0.114f * b;
+// shaders/ssim/ssim_lumapack.glsl:19-21 (G weight 0.581 as in the reference) times 255000: at most 253470.
+__device__ __forceinline__ int luma_i(uint32_t px, int add) {
+    return int(__dp2a_hi(114u, px, __dp2a_lo(299u | 581u << 16, px, unsigned(add))));
 }
+// (u, v) of a pixel pair as 1.5 * 2^23 + value in floats, whose spacing there is 1
+__device__ __forceinline__ float2 uv_biased(uint32_t pa, uint32_t pb) {
+    const int a = luma_i(pa, 0x4B400000), b = luma_i(pb, 0);
+    return make_float2(__int_as_float(a + b), __int_as_float(a - b));
+}
+constexpr float UV_BIAS = 12582912.0f;
 
 __device__ __forceinline__ int find_pair(const SsimPairDev *pairs, int n, int tile) {
     int lo = 0, hi = n - 1;
@@ -91,70 +96,14 @@ __device__ __forceinline__ int find_pair(const SsimPairDev *pairs, int n, int ti
     return lo;
 }
 
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, int src_bytes) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-// "memory" clobbers: the compiler must not move shared-memory accesses across the copies or waits
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-// Issue the copies of image row y (both images, staged columns) into raw ring slot `slot`.
-// Columns or rows outside the image are not fetched: the conversion step zeroes them.
-__device__ __forceinline__ void issue_row(Smem &sm, const SsimPairDev &P, int x0, int y, int slot) {
-    if (y < 0 || y >= P.h) return;
-    const int xs = x0 - 8;
-    if (P.vec_ok) {
-        constexpr int CH = SMEM_COLS / 4;  // 16-byte chunks per image row
-        for (int c = threadIdx.x; c < 2 * CH; c += NT) {
-            const int img = c / CH, q = c - img * CH;
-            const int x = xs + 4 * q;
-            if (x < 0 || x >= P.w) continue;
-            const int valid = min(4, P.w - x);
-            const uint8_t *src = (img ? P.b : P.a) + (long long)y * P.pitch + 4LL * x;
-            cp_async16(&sm.raw[slot][img][4 * q], src, 4 * valid);
-        }
-    } else {
-        for (int c = threadIdx.x; c < 2 * SMEM_COLS; c += NT) {
-            const int img = c / SMEM_COLS, q = c - img * SMEM_COLS;
-            const int x = xs + q;
-            if (x < 0 || x >= P.w) continue;
-            const uint8_t *src = (img ? P.b : P.a) + (long long)y * P.pitch + 4LL * x;
-            cp_async4(&sm.raw[slot][img][q], src);
-        }
-    }
-}
-
-// Raw RGBA row -> shifted (u, v) row; positions outside the image become (0, 0), which removes
-// them from every window sum (the reference skips out-of-image taps).
-__device__ __forceinline__ void convert_row(Smem &sm, const SsimPairDev &P, int x0, int y, int slot,
-                                            float2 *dst, float cu, float cv) {
-    const bool row_ok = y >= 0 && y < P.h;
-    for (int q = threadIdx.x; q < SMEM_COLS; q += NT) {
-        const int x = x0 - 8 + q;
-        float2 o = make_float2(0.f, 0.f);
-        if (row_ok && x >= 0 && x < P.w) {
-            const float la = luma_u8(sm.raw[slot][0][q]), lb = luma_u8(sm.raw[slot][1][q]);
-            o = make_float2((la + lb) - cu, (la - lb) - cv);
-        }
-        dst[q] = o;
-    }
-}
-
-// Deterministic pooling, shared by the SSIM kernels: the CTA's partial (FP64, fixed order) goes to
+// Deterministic pooling: the CTA's partial (FP64, fixed order) goes to
 // its tile slot; the last CTA of the pair to finish sums the pair's slots in a fixed order and
 // writes the mean (`count` pooled pixels).  `red` holds NTH/32 doubles of shared memory.
 template <int NTH>
-__device__ __forceinline__ void pool_tiles(float acc, double *red, int *is_last, double *partials,
+__device__ __forceinline__ void pool_tiles(double d, double *red, int *is_last, double *partials,
                                            unsigned *counters, double *scores, int pi, const SsimPairDev &P,
                                            int gt, double count) {
     const int tid = threadIdx.x;
-    double d = double(acc);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
     if ((tid & 31) == 0) red[tid >> 5] = d;
@@ -187,12 +136,66 @@ __device__ __forceinline__ void pool_tiles(float acc, double *red, int *is_last,
     }
 }
 
+// One thread's share of the staging: a 4-pixel chunk of both images in one row of every step.
+struct Chunk {
+    const uint8_t *a, *b;  // the chunk in the next step's row
+    int y;                 // that row
+    int nv;                // pixels of the chunk inside the image's columns
+    int at;                // its first unit in Smem::uv
+    uint4 ra, rb;
+
+    __device__ __forceinline__ void init(const SsimPairDev &P, int xs, int yr, int c) {
+        const int row = c / CHUNKS, q = c - row * CHUNKS, x = xs + 4 * q;
+        y = yr + row;
+        nv = x < 0 ? 0 : max(0, min(4, P.w - x));  // x is a multiple of 4: a chunk is all left of 0 or not at all
+        a = P.a + (long long)y * P.pitch + 4LL * x;
+        b = P.b + (long long)y * P.pitch + 4LL * x;
+        at = row * UNITS + 2 * q;
+    }
+    // Reads the chunk (pixels outside the image are not read) and moves on to the next step's row.
+    __device__ __forceinline__ void load(const SsimPairDev &P) {
+        if (unsigned(y) < unsigned(P.h)) {
+            if (P.vec_ok && nv == 4) {
+                ra = __ldg(reinterpret_cast<const uint4 *>(a));
+                rb = __ldg(reinterpret_cast<const uint4 *>(b));
+            } else {
+                const uint32_t *pa = reinterpret_cast<const uint32_t *>(a), *pb = reinterpret_cast<const uint32_t *>(b);
+                if (nv > 0) ra.x = __ldg(pa), rb.x = __ldg(pb);
+                if (nv > 1) ra.y = __ldg(pa + 1), rb.y = __ldg(pb + 1);
+                if (nv > 2) ra.z = __ldg(pa + 2), rb.z = __ldg(pb + 2);
+                if (nv > 3) ra.w = __ldg(pa + 3), rb.w = __ldg(pb + 3);
+            }
+        }
+        a += RSTEP * P.pitch;
+        b += RSTEP * P.pitch;
+        y += RSTEP;
+    }
+    // Stores the shifted (u, v) of what was read; pixels outside the image become (0, 0), which removes
+    // them from every window sum (the reference skips out-of-image taps).
+    __device__ __forceinline__ void store(Smem &sm, int h, float2 shift) const {
+        float2 v[4] = {__fadd2_rn(uv_biased(ra.x, rb.x), shift), __fadd2_rn(uv_biased(ra.y, rb.y), shift),
+                       __fadd2_rn(uv_biased(ra.z, rb.z), shift), __fadd2_rn(uv_biased(ra.w, rb.w), shift)};
+        const int n = unsigned(y - RSTEP) < unsigned(h) ? nv : 0;
+        if (n < 4) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k >= n) v[k] = make_float2(0.f, 0.f);
+        }
+        float4 *uv = &sm.uv[0][0];
+        uv[unit_at(at)] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+        uv[unit_at(at + 1)] = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
+    }
+};
+
+// Bound by the FMA pipe (60% busy) and instruction issue (58%): 144 instructions a pixel pair, of which 47
+// are the packed taps of both passes.  Four CTAs per SM at 124 registers, 16 1080p pairs: 236 us, against
+// 397 us for the form before it (a column a thread, eleven loads and squares per pixel, the row loop
+// unrolled over the window, a barrier a row; 297 instructions a pixel pair); five CTAs at 96 registers
+// spill, 253 us.  The split-precision tensor-core form took 23.1 us a 1080p pair and the single-product
+// one 15.6 us where this takes 14.7, so every form asked for computes here.
 template <int R>
-// 8 CTAs of 128 threads per SM (at most 64 registers a thread): the row pipeline is latency-bound,
-// so resident warps matter more than registers per thread.
-__global__ void __launch_bounds__(NT, 8) ssim_kernel(SsimArgs args) {
-    using G = Geom<R>;
-    constexpr int K = G::K, S = G::S, ROWS = G::ROWS;
+__global__ void __launch_bounds__(NT, 4) ssim_kernel(SsimArgs args) {
+    constexpr int K = 2 * R + 1;
     __shared__ __align__(16) Smem sm;
     __shared__ double red[NT / 32];
     __shared__ int is_last;
@@ -202,140 +205,137 @@ __global__ void __launch_bounds__(NT, 8) ssim_kernel(SsimArgs args) {
     const SsimPairDev P = args.pairs[pi];
     const int local = gt - P.tile_base;
     const int x0 = (local % P.tiles_x) * TW;
-    const int y0 = (local / P.tiles_x) * S;
-    const int W = P.w, H = P.h;
-    const int tid = threadIdx.x;
+    const int y0 = (local / P.tiles_x) * args.strip;
+    const int W = P.w, H = P.h, xs = x0 - 8;
+    const int y1 = min(y0 + args.strip, H);  // end of the strip's output rows
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    // prefetch the first PF rows (tile row r = image row y0 - R + r)
-#pragma unroll
-    for (int r = 0; r < PF; r++) {
-        issue_row(sm, P, x0, y0 - R + r, r % NRAW);
-        cp_async_commit();
-    }
-
-    // per-tile shift constants: u, v of the tile's centre pixel (keeps FP32 cancellation small)
-    float cu, cv;
+    // the strip's shift constants: u, v of the centre pixel of its block of SHIFT_ROWS rows
+    float2 shift, c;
     {
-        const int cx = min(x0 + TW / 2, W - 1), cy = min(y0 + S / 2, H - 1);
-        const uint32_t pa = __ldg(reinterpret_cast<const uint32_t *>(P.a + (long long)cy * P.pitch) + cx);
-        const uint32_t pb = __ldg(reinterpret_cast<const uint32_t *>(P.b + (long long)cy * P.pitch) + cx);
-        const float la = luma_u8(pa), lb = luma_u8(pb);
-        cu = la + lb;
-        cv = la - lb;
+        const int cx = min(x0 + TW / 2, W - 1), cy = min((y0 & ~(SHIFT_ROWS - 1)) + SHIFT_ROWS / 2, H - 1);
+        shift = uv_biased(__ldg(reinterpret_cast<const uint32_t *>(P.a + (long long)cy * P.pitch) + cx),
+                          __ldg(reinterpret_cast<const uint32_t *>(P.b + (long long)cy * P.pitch) + cx));
+        c = make_float2(shift.x - UV_BIAS, shift.y - UV_BIAS);
+        shift = make_float2(-shift.x, -shift.y);
     }
-
-    cp_async_wait<PF - 1>();
-    __syncthreads();
-    convert_row(sm, P, x0, y0 - R, 0, sm.uv[0], cu, cv);
-    issue_row(sm, P, x0, y0 - R + PF, PF % NRAW);
-    cp_async_commit();
-
-    const int col0 = tid;                // this thread's tile column
-    const int start = col0 + 8 - R;      // staged index of its leftmost horizontal tap
-    float gsum = 0.f;
-#pragma unroll
-    for (int k = 0; k < K; k++) gsum += args.g[k];
-    constexpr int CPT = 1;
-    float rwx[CPT];
-#pragma unroll
-    for (int c = 0; c < CPT; c++) {
-        const int x = x0 + col0 + c;
+    auto tap = [&](int k) { return args.g[k < R ? R - k : k - R]; };  // g(k - R), symmetric
+    const int x = x0 + tid;  // this thread's column of the vertical pass
+    float rwx;               // 1 / in-image weight of the horizontal window
+    {
         float s = 0.f;
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-            const int xx = x + k - R;
-            s += (xx >= 0 && xx < W) ? args.g[k] : 0.f;
-        }
-        rwx[c] = 1.0f / s;
+        for (int k = 0; k < K; k++) s += (x + k - R >= 0 && x + k - R < W) ? tap(k).x : 0.f;
+        rwx = 1.0f / s;
     }
+    float gsum = args.g[0].x;
+#pragma unroll
+    for (int k = 1; k <= R; k++) gsum += 2.0f * args.g[k].x;
+    const bool pool_x = x >= R && x <= W - R && x < W;
 
-    float2 ring_m[CPT][K];  // (sum g u, sum g v) of the last K rows, per column
-    float2 ring_s[CPT][K];  // (sum g u^2, sum g v^2)
-    float acc = 0.f;      // pooled SSIM of this thread
-    bool col_in[CPT];
+    float2 am[K - 1], as[K - 1];  // running vertical sums: element k waits for K - 1 - k more rows
 #pragma unroll
-    for (int c = 0; c < CPT; c++) col_in[c] = x0 + col0 + c < W;
+    for (int k = 0; k < K - 1; k++) am[k] = as[k] = make_float2(0.f, 0.f);
+    float acc = 0.f;     // pooled SSIM of up to four rows
+    long long sum = 0;   // and of the strip, in units of 2^-26
+    double other = 0.0;  // sums that are no such numbers: k1 or k2 of 0 over flat areas
+    auto pool = [&] {
+        if (fabsf(acc) < 16.0f) sum += __float2int_rn(acc * 67108864.0f);
+        else other += acc;
+        acc = 0.f;
+    };
 
-    for (int jb = 0; jb < ROWS; jb += K) {
-#pragma unroll
-        for (int t = 0; t < K; t++) {
-            const int j = jb + t;
-            // make row j+1 available: wait for its copies, convert it, prefetch row j+1+PF
-            cp_async_wait<PF - 1>();
-            __syncthreads();
-            if (j + 1 < ROWS) convert_row(sm, P, x0, y0 - R + j + 1, (j + 1) % NRAW, sm.uv[(j + 1) & 1], cu, cv);
-            if (j + 1 + PF < ROWS) issue_row(sm, P, x0, y0 - R + j + 1 + PF, (j + 1 + PF) % NRAW);
-            cp_async_commit();
+    const int yr = y0 - R;  // image row of the first staged row
+    const int steps = (y1 - y0 + 2 * R + RSTEP - 1) / RSTEP;
+    constexpr int EXTRA = RSTEP * CHUNKS - NT;  // chunks beyond one a thread
+    Chunk first, second;
+    first.init(P, xs, yr, tid);
+    first.load(P);
+    if (tid < EXTRA) {
+        second.init(P, xs, yr, NT + tid);
+        second.load(P);
+    }
+    first.store(sm, H, shift);
+    if (tid < EXTRA) second.store(sm, H, shift);
+    __syncthreads();
 
-            // horizontal taps of row j
-            float2 v[K];
+#pragma unroll 1
+    for (int s = 0; s < steps; s++) {
+        if (s + 1 < steps) {  // the next step's pixels arrive under this step's taps
+            first.load(P);
+            if (tid < EXTRA) second.load(P);
+        }
+        {
+            // horizontal taps of row `warp`, columns 4 lane .. 4 lane + 3: staged columns 4 lane + 8 - R ..
+            float2 hm[4], hs[4];
 #pragma unroll
-            for (int q = 0; q < K; q++) v[q] = sm.uv[j & 1][start + q];
+            for (int j = 0; j < 4; j++) hm[j] = hs[j] = make_float2(0.f, 0.f);
+            constexpr int U0 = (8 - R) / 2, U1 = (8 + 3 + R) / 2;
 #pragma unroll
-            for (int c = 0; c < CPT; c++) {
-                float2 hm = make_float2(0.f, 0.f), hs = make_float2(0.f, 0.f);
+            for (int u = U0; u <= U1; u++) {
+                const float4 two = (&sm.uv[0][0])[unit_at(warp * UNITS + 2 * lane + u)];
 #pragma unroll
-                for (int k = 0; k < K; k++) {
-                    const float2 sv = v[c + k];
-                    const float2 gs = __fmul2_rn(make_float2(args.g[k], args.g[k]), sv);
-                    hm = __fadd2_rn(hm, gs);
-                    hs = __ffma2_rn(gs, sv, hs);
-                }
-                ring_m[c][t] = hm;
-                ring_s[c][t] = hs;
-            }
-            if (j >= 2 * R) {
-                // vertical taps: output row i = j - 2R uses tile rows i .. i + 2R
-                const int y = y0 + j - 2 * R;
-                if (y < H) {
-                    float wy = gsum;
-                    if (y < R || y >= H - R) {
-                        wy = 0.f;
+                for (int e = 0; e < 2; e++) {
+                    const int i = 2 * u + e - (8 - R);  // tap of column 0
+                    if (i < 0 || i > K + 2) continue;
+                    const float2 v = e ? make_float2(two.z, two.w) : make_float2(two.x, two.y);
+                    const float2 q = __fmul2_rn(v, v);
 #pragma unroll
-                        for (int k = 0; k < K; k++) {
-                            const int yy = y + k - R;
-                            wy += (yy >= 0 && yy < H) ? args.g[k] : 0.f;
-                        }
-                    }
-                    const float rwy = 1.0f / wy;
-                    const bool pool_y = y >= R && y <= H - R;
-#pragma unroll
-                    for (int c = 0; c < CPT; c++) {
-                        float2 mm = make_float2(0.f, 0.f), ms = make_float2(0.f, 0.f);
-#pragma unroll
-                        for (int k = 0; k < K; k++) {
-                            const int slot = (t + 1 + k) % K;
-                            const float2 gk = make_float2(args.g[k], args.g[k]);
-                            mm = __ffma2_rn(gk, ring_m[c][slot], mm);
-                            ms = __ffma2_rn(gk, ring_s[c][slot], ms);
-                        }
-                        if (col_in[c]) {
-                            const int x = x0 + col0 + c;
-                            const float inv = rwx[c] * rwy;
-                            const float su = mm.x * inv, sv = mm.y * inv;  // shifted means
-                            const float varu = fmaf(ms.x, inv, -su * su);
-                            const float varv = fmaf(ms.y, inv, -sv * sv);
-                            const float mu = su + cu, mv = sv + cv;
-                            const float mu2 = mu * mu, mv2 = mv * mv;
-                            const float num = (0.5f * (mu2 - mv2) + args.c1) * (0.5f * (varu - varv) + args.c2);
-                            const float den = (0.5f * (mu2 + mv2) + args.c1) * (0.5f * (varu + varv) + args.c2);
-                            const float ssim = num * iqm::rcp_approx(den);  // den >= c1 c2 > 0
-                            if (P.map) P.map[(long long)y * W + x] = ssim;
-                            if (pool_y && x >= R && x <= W - R) acc += ssim;
-                        }
+                    for (int j = 0; j < 4; j++) {
+                        if (i - j < 0 || i - j >= K) continue;
+                        hm[j] = i == j ? __fmul2_rn(tap(0), v) : __ffma2_rn(tap(i - j), v, hm[j]);
+                        hs[j] = i == j ? __fmul2_rn(tap(0), q) : __ffma2_rn(tap(i - j), q, hs[j]);
                     }
                 }
             }
+#pragma unroll
+            for (int j = 0; j < 4; j++) sm.h[warp][column_at(4 * lane + j)] = make_float4(hm[j].x, hm[j].y, hs[j].x, hs[j].y);
         }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < RSTEP; i++) {
+            const float4 h = sm.h[i][column_at(tid)];
+            const float2 h1 = make_float2(h.x, h.y), h2 = make_float2(h.z, h.w);
+            const float2 mm = __ffma2_rn(tap(K - 1), h1, am[0]), ms = __ffma2_rn(tap(K - 1), h2, as[0]);
+#pragma unroll
+            for (int k = 0; k < K - 2; k++) {
+                am[k] = __ffma2_rn(tap(K - 2 - k), h1, am[k + 1]);
+                as[k] = __ffma2_rn(tap(K - 2 - k), h2, as[k + 1]);
+            }
+            am[K - 2] = __fmul2_rn(tap(0), h1);
+            as[K - 2] = __fmul2_rn(tap(0), h2);
+            const int y = yr + RSTEP * s + i - R;  // the output row that this row completes
+            if (y < y0 || y >= y1) continue;       // uniform
+            float wy = gsum;
+            if (y < R || y >= H - R) {
+                wy = 0.f;
+#pragma unroll
+                for (int k = 0; k < K; k++) wy += (y + k - R >= 0 && y + k - R < H) ? tap(k).x : 0.f;
+            }
+            const float inv = rwx * iqm::rcp_approx(wy);
+            const float2 sh = __fmul2_rn(mm, make_float2(inv, inv));  // shifted means
+            const float varu = fmaf(ms.x, inv, -sh.x * sh.x), varv = fmaf(ms.y, inv, -sh.y * sh.y);
+            const float2 mu = __fadd2_rn(sh, c), mu2 = __fmul2_rn(mu, mu);
+            const float num = fmaf(0.5f, mu2.x - mu2.y, args.c1) * fmaf(0.5f, varu - varv, args.c2);
+            const float den = fmaf(0.5f, mu2.x + mu2.y, args.c1) * fmaf(0.5f, varu + varv, args.c2);
+            const float ssim = num * iqm::rcp_approx(den);  // den >= c1 c2 > 0
+            if (P.map && x < W) P.map[(long long)y * W + x] = ssim;
+            if (y >= R && y <= H - R) acc += pool_x ? ssim : 0.f;
+            if (((i - 2 * R) & 3) == 3) pool();  // y & 3 == 3: strips start at multiples of 4
+        }
+        if (s + 1 < steps) {
+            first.store(sm, H, shift);
+            if (tid < EXTRA) second.store(sm, H, shift);
+        }
+        __syncthreads();
     }
-    cp_async_wait<0>();
-    pool_tiles<NT>(acc, red, &is_last, args.partials, args.counters, args.scores, pi, P, gt,
+    pool();
+    // Sums of these are exact in FP64 (up to 2^27 pixels), so their order does not matter.
+    pool_tiles<NT>(double(sum) * (1.0 / 67108864.0) + other, red, &is_last, args.partials, args.counters, args.scores, pi, P, gt,
                    double(W - 2 * R + 1) * double(H - 2 * R + 1));
 }
 
 }  // namespace
-
-#include "ssim_mma.cuh"
 
 namespace {
 
@@ -344,16 +344,24 @@ void launch_ssim(const SsimArgs &a, int total_tiles, cudaStream_t s) {
     ssim_kernel<R><<<total_tiles, NT, 0, s>>>(a);
 }
 
-int strip_rows(int R) {
-    switch (R) {
-        case 1: return Geom<1>::S;
-        case 2: return Geom<2>::S;
-        case 3: return Geom<3>::S;
-        case 4: return Geom<4>::S;
-        case 5: return Geom<5>::S;
-        case 6: return Geom<6>::S;
-        default: return Geom<7>::S;
+// Rows of a tile, the same for all pairs of a launch: the power of two that divides SHIFT_ROWS with the
+// least estimated time, a tile's rows with its halo (and about a dozen rows' worth of set-up) times the
+// rounds of two CTAs per SM that it takes.  The values of an image do not depend on the choice.  Strips
+// of 8 / 16 / 32 / 64 / 128 rows: one 512x512 pair 15.2 / 15.5 / 19.6 / 27.5 / 43.5 us, 16 1080p pairs
+// 504 / 350 / 273 / 238 / 236 us.
+int strip_rows(const iqm_pair *pairs, int n, int R) {
+    int best = SHIFT_ROWS;
+    double best_cost = 0.0;
+    for (int s = SHIFT_ROWS; s >= 8; s /= 2) {
+        double tiles = 0.0;
+        for (int i = 0; i < n; i++) tiles += double(iqm::ceil_div(pairs[i].w, TW)) * iqm::ceil_div(pairs[i].h, s);
+        const double cost = (s + 2 * R + 12) * std::max(1.0, tiles / (2 * 148));
+        if (s == SHIFT_ROWS || cost < best_cost) {
+            best = s;
+            best_cost = cost;
+        }
     }
+    return best;
 }
 
 void check_params(const iqm_ssim_params &p) {
@@ -365,18 +373,14 @@ void check_params(const iqm_ssim_params &p) {
                 "unknown precision " + std::to_string(p.precision));
 }
 
-// The tensor-core kernel (one 64x32 tile per CTA) for IQM_MIXED (split products) and
-// IQM_MIXED_FAST (single products).
-// Persistent launch: as many CTAs as fit on the device at once (at most one per work unit).
-template <int SPLIT>
-void launch_ssim_mma(const SsimMmaArgs &a, int total_units, int device, cudaStream_t s) {
-    const size_t smem = SsimMmaGeom<SPLIT>::smem_bytes;
-    IQM_CHECK_CUDA(cudaFuncSetAttribute(ssim_mma_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int sms = 0, per_sm = 0;
-    IQM_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    IQM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ssim_mma_kernel<SPLIT>, MT_THREADS, smem));
-    const int grid = std::max(1, std::min(total_units, sms * std::max(1, per_sm)));
-    ssim_mma_kernel<SPLIT><<<grid, MT_THREADS, smem, s>>>(a, total_units);
+// Taps and constants of the kernel.
+void set_constants(SsimArgs &a, const iqm_ssim_params &p, int R) {
+    for (int k = 0; k < 8; k++) {
+        const float g = k <= R ? float(std::exp(-double(k * k) / (2.0 * double(p.sigma) * p.sigma))) : 0.f;
+        a.g[k] = make_float2(g, g);
+    }
+    a.c1 = p.k1 * p.k1 * (LUMA_UNIT * LUMA_UNIT);
+    a.c2 = p.k2 * p.k2 * (LUMA_UNIT * LUMA_UNIT);
 }
 
 // Enqueue SSIM for device-resident pairs; `maps[i]` (device, nullable) receive the SSIM maps.
@@ -384,11 +388,9 @@ void ssim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, const iqm_ss
                   const std::vector<float *> &maps, double *d_scores) {
     const int n = int(pairs.size());
     const int R = (p.kernel_size - 1) / 2;
-    const bool mma = p.precision != IQM_FP32;
-    const int tw = mma ? MT_W : TW, th = mma ? MT_H : strip_rows(R);
+    const int strip = strip_rows(pairs.data(), n, R);
     std::vector<SsimPairDev> hd(n);
-    int total = 0, units = 0;
-    const int segt = MT_SEG_SPLIT;  // tensor-core kernel: tiles per column segment (work unit)
+    int total = 0;
     for (int i = 0; i < n; i++) {
         const iqm_pair &q = pairs[i];
         SsimPairDev &d = hd[i];
@@ -398,50 +400,29 @@ void ssim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, const iqm_ss
         d.pitch = (long long)q.row_bytes;
         d.w = q.w;
         d.h = q.h;
-        d.tiles_x = int(iqm::ceil_div(q.w, tw));
-        d.ntiles = d.tiles_x * int(iqm::ceil_div(q.h, th));
+        d.tiles_x = int(iqm::ceil_div(q.w, TW));
+        d.ntiles = d.tiles_x * int(iqm::ceil_div(q.h, strip));
         d.tile_base = total;
         d.vec_ok = ((reinterpret_cast<uintptr_t>(q.input) | reinterpret_cast<uintptr_t>(q.ref) |
                      uintptr_t(q.row_bytes)) & 15u) == 0;
-        d.unit_base = units;
         total += d.ntiles;
-        units += d.tiles_x * int(iqm::ceil_div(d.ntiles / d.tiles_x, segt));
     }
     auto *d_desc = static_cast<SsimPairDev *>(
         iqm::upload_bytes(ctx, ctx->desc, hd.data(), sizeof(SsimPairDev) * n));
     const size_t part_bytes = (sizeof(double) * total + 255) & ~size_t(255);
     const size_t cnt_bytes = (sizeof(unsigned) * n + 255) & ~size_t(255);
     auto *scr = static_cast<uint8_t *>(ctx->scratch.get(part_bytes + cnt_bytes, ctx->stream));
-    double g64[15] = {}, gsum = 0.0;
-    for (int k = -R; k <= R; k++) gsum += (g64[k + R] = std::exp(-double(k * k) / (2.0 * double(p.sigma) * p.sigma)));
     auto *counters = reinterpret_cast<unsigned *>(scr + part_bytes);
     IQM_CHECK_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned) * n, ctx->stream));
     iqm::timing_mark(ctx, nullptr);
-    if (mma) {
-        SsimMmaArgs a{};
-        a.pairs = d_desc;
-        a.npairs = n;
-        a.R = R;
-        a.partials = reinterpret_cast<double *>(scr);
-        a.counters = counters;
-        a.scores = d_scores;
-        for (int k = 0; k < 15; k++) a.gn[k] = float(g64[k] / gsum);
-        a.c1 = p.k1 * p.k1;
-        a.c2 = p.k2 * p.k2;
-        if (p.precision == IQM_MIXED) launch_ssim_mma<3>(a, units, ctx->device, ctx->stream);
-        else launch_ssim_mma<1>(a, units, ctx->device, ctx->stream);
-        iqm::check_launch(ctx, "ssim_mma_kernel");
-        return;
-    }
     SsimArgs a{};
     a.pairs = d_desc;
     a.npairs = n;
     a.partials = reinterpret_cast<double *>(scr);
     a.counters = counters;
     a.scores = d_scores;
-    for (int k = 0; k < 15; k++) a.g[k] = float(g64[k]);
-    a.c1 = p.k1 * p.k1;
-    a.c2 = p.k2 * p.k2;
+    a.strip = strip;
+    set_constants(a, p, R);
     switch (R) {
         case 1: launch_ssim<1>(a, total, ctx->stream); break;
         case 2: launch_ssim<2>(a, total, ctx->stream); break;
@@ -591,8 +572,15 @@ extern "C" __attribute__((visibility("default"))) int iqm_ssim_noalloc(
     const int R = (p.kernel_size - 1) / 2;
     if (w < 2 * R || h < 2 * R || w > 65536 || h > 65536 || row_bytes < size_t(w) * 4) return IQM_EINVAL;
     const int tiles_x = int(iqm::ceil_div(w, TW));
-    const long tiles = long(tiles_x) * long(iqm::ceil_div(h, strip_rows(R)));
-    if (tiles > IQM_SSIM_NOALLOC_MAX_TILES) return IQM_EINVAL;
+    // the documented bound is in tiles of 120 to 127 rows (the 2R + 1 rows of a window divide a tile and
+    // its halo); the kernel's own tiles of SHIFT_ROWS rows are never more
+    const int bound_rows = (2 * R + 1) * int(iqm::ceil_div(120 + 2 * R, 2 * R + 1)) - 2 * R;
+    if (long(tiles_x) * long(iqm::ceil_div(h, bound_rows)) > IQM_SSIM_NOALLOC_MAX_TILES) return IQM_EINVAL;
+    // shorter strips for small images, as iqm_ssim takes them, while their sums fit the scratch
+    const iqm_pair one{d_in, d_ref, w, h, row_bytes};
+    int strip = strip_rows(&one, 1, R);
+    while (strip < SHIFT_ROWS && long(tiles_x) * long(iqm::ceil_div(h, strip)) > IQM_SSIM_NOALLOC_MAX_TILES) strip *= 2;
+    const long tiles = long(tiles_x) * long(iqm::ceil_div(h, strip));
 
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= NOALLOC_MAX_DEVICES) return IQM_ECUDA;
@@ -640,10 +628,8 @@ extern "C" __attribute__((visibility("default"))) int iqm_ssim_noalloc(
     a.partials = s->partials;
     a.counters = &s->counter;
     a.scores = d_mssim;
-    for (int k = 0; k < 15; k++) a.g[k] = 0.f;
-    for (int k = -R; k <= R; k++) a.g[k + R] = float(std::exp(-double(k * k) / (2.0 * double(p.sigma) * p.sigma)));
-    a.c1 = p.k1 * p.k1;
-    a.c2 = p.k2 * p.k2;
+    a.strip = strip;
+    set_constants(a, p, R);
     cudaError_t e;
     switch (R) {
         case 1: e = launch_ssim_checked<1>(a, int(tiles), st); break;
