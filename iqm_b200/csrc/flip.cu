@@ -7,29 +7,22 @@
 // pow(dEc, 1 - dEf) is never read back or pooled (FLIPResult::mean_flip is never set); the score
 // here is its mean.
 //
-// Two kernels:
-//   flip_hpass_kernel  one CTA per 512-pixel segment of 8 rows of both images, walked row by row
-//                      with each row's pixels loaded during the previous row's taps (measured
-//                      1.41x the one-row-per-CTA form at 67 ppd): RGBA8 -> linear RGB by a
+// One kernel for filter radii up to 14 (about 103 pixels per degree), flip_kernel: both filter passes and the
+// per-pixel error of a strip of columns, nothing between them leaving the SM.  Wider filters take two:
+//   flip_hpass_kernel  one CTA per 512-pixel segment of 8 rows of both images, walked row by row with each
+//                      row's pixels loaded during the previous row's taps: RGBA8 -> linear RGB by a
 //                      256-entry table (the sRGB curve of srgb_to_ycxcz.glsl:22-28 on 8-bit inputs),
 //                      -> XYZ -> YCxCz in shared memory, then the horizontal feature taps (g, edge,
 //                      point on (Y+16)/116, feature_filter_horizontal.glsl) and the horizontal CSF
-//                      taps (spatial_prefilter_horizontal.glsl), clamp-to-edge; 4 pixels per thread;
-//                      12 planes out;
-//   flip_vcols_kernel  (radii known at compile time) 32-column strips, one warp per (image, plane,
-//                      filter) role walking down the strip with a (2R+1)-row register window, the
-//                      14 filtered values per pixel exchanged through shared memory; or
-//   flip_vpass_kernel  (any radii) 32x32-pixel output tiles: the 12 planes (+ halo rows, clamp-to-edge)
-//                      staged in shared memory, vertical feature and CSF taps register-blocked 8 rows
-//                      per thread; both then YCxCz -> XYZ -> linear RGB (clamped) -> L*a*b* -> Hunt
-//                      (spatial_prefilter.glsl:74-99), HyAB colour error (spatial_detection.glsl),
-//                      feature error (feature_detection.glsl:48-53), combine
-//                      (combine_error_maps.glsl:28) and FP64 pooling; the last CTA of a pair writes
-//                      the mean.
+//                      taps (spatial_prefilter_horizontal.glsl), clamp-to-edge; 12 planes out;
+//   flip_vpass_kernel  32x32-pixel output tiles: the 12 planes (+ halo rows, clamp-to-edge) staged in
+//                      shared memory, vertical feature and CSF taps register-blocked 8 rows per thread.
+// All end with YCxCz -> XYZ -> linear RGB (clamped) -> L*a*b* -> Hunt (spatial_prefilter.glsl:74-99), HyAB
+// colour error (spatial_detection.glsl), feature error (feature_detection.glsl:48-53), combine
+// (combine_error_maps.glsl:28) and FP64 pooling; the last CTA of a pair writes the mean.
 // Filter taps depend only on pixels-per-degree: computed on the host in double, normalised once.
-// Both images go through the same compiled code (the per-pixel colour math works on float2 pairs
-// {input, reference} with packed FP32x2 instructions, the row pass is one loop), so identical
-// images give exactly 0.
+// Both images go through the same compiled code (float2 pairs {input, reference} with packed FP32x2
+// instructions, or one loop over both), so identical images give exactly 0.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -82,6 +75,7 @@ struct FlipArgs {
     unsigned *counters;
     double *scores;
     long long total_segs;
+    int strip;  // rows of a tile (flip_kernel)
 };
 
 __device__ __forceinline__ int find_seg(const FlipPairDev *p, int n, long long s) {
@@ -108,9 +102,6 @@ using iqm::fma2;
 using iqm::mul2;
 using iqm::sub2;
 
-// RF, RC > 0: filter radii fixed at compile time (tap loops unrolled, weights as constant-bank
-// operands); 0: read from T.
-template <int RF, int RC>
 __global__ void __launch_bounds__(HT, 8) flip_hpass_kernel(FlipArgs args, const __grid_constant__ FlipTaps T) {
     __shared__ float lin[256];
     __shared__ float ycc[2][4][HSEG + 2 * MAXR];  // Y, Cx, Cz and (Y + 16) / 116
@@ -122,7 +113,7 @@ __global__ void __launch_bounds__(HT, 8) flip_hpass_kernel(FlipArgs args, const 
     const int y_first = int(local / segs_x) * HROWS;
     const int y_end = min(y_first + HROWS, P.h);
     const int x0 = int(local % segs_x) * HSEG;
-    const int rf = RF ? RF : T.rf, rc = RC ? RC : T.rc;
+    const int rf = T.rf, rc = T.rc;
     const int R = max(rf, rc);
     for (int i = threadIdx.x; i < 256; i += HT) lin[i] = T.lin[i];
     // columns x0-R .. x0+HSEG+R-1 (clamped to the image) of both images; each thread's share of a
@@ -172,61 +163,23 @@ __global__ void __launch_bounds__(HT, 8) flip_hpass_kernel(FlipArgs args, const 
     for (int img = 0; img < 2; img++) {
         float fa[4][3] = {}, ca[4][3] = {};
         // output column x = x0 + xl + i, tap j, reads staged column xl + i + u with u = R - j
-        if constexpr (RF > 0) {
-            // radii known: slide a 4-wide register window along u (one new value per plane per tap)
-            constexpr int RR = RF > RC ? RF : RC;
-            float win[4][4];
+        for (int j = -R; j <= R; j++) {
+            const bool uf = j >= -rf && j <= rf, uc = j >= -rc && j <= rc;
+            const float wg = uf ? T.feat[0][j + rf] : 0.f, we = uf ? T.feat[1][j + rf] : 0.f,
+                        wp = uf ? T.feat[2][j + rf] : 0.f;
+            const float w0 = uc ? T.csf[0][j + rc] : 0.f, w1 = uc ? T.csf[1][j + rc] : 0.f,
+                        w2 = uc ? T.csf[2][j + rc] : 0.f;
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-#pragma unroll
-                for (int i = 0; i < 3; i++) win[q][i + 1] = ycc[img][q][xl + i];
-#pragma unroll
-            for (int u = 0; u <= 2 * RR; u++) {
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-#pragma unroll
-                    for (int i = 0; i < 3; i++) win[q][i] = win[q][i + 1];
-                    win[q][3] = ycc[img][q][xl + u + 3];
-                }
-                const int j = RR - u;
-                if (j >= -RF && j <= RF) {
-                    const float wg = T.feat[0][j + RF], we = T.feat[1][j + RF], wp = T.feat[2][j + RF];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        fa[i][0] = fmaf(we, win[3][i], fa[i][0]);  // dx   (edge)
-                        fa[i][1] = fmaf(wp, win[3][i], fa[i][1]);  // ddx  (point)
-                        fa[i][2] = fmaf(wg, win[3][i], fa[i][2]);  // value (gauss)
-                    }
-                }
-                if (j >= -RC && j <= RC) {
-                    const float w0 = T.csf[0][j + RC], w1 = T.csf[1][j + RC], w2 = T.csf[2][j + RC];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        ca[i][0] = fmaf(w0, win[0][i], ca[i][0]);
-                        ca[i][1] = fmaf(w1, win[1][i], ca[i][1]);
-                        ca[i][2] = fmaf(w2, win[2][i], ca[i][2]);
-                    }
-                }
-            }
-        } else {
-            for (int j = -R; j <= R; j++) {
-                const bool uf = j >= -rf && j <= rf, uc = j >= -rc && j <= rc;
-                const float wg = uf ? T.feat[0][j + rf] : 0.f, we = uf ? T.feat[1][j + rf] : 0.f,
-                            wp = uf ? T.feat[2][j + rf] : 0.f;
-                const float w0 = uc ? T.csf[0][j + rc] : 0.f, w1 = uc ? T.csf[1][j + rc] : 0.f,
-                            w2 = uc ? T.csf[2][j + rc] : 0.f;
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int c = xl + i - j + R;
-                    const float Yv = ycc[img][0][c];
-                    const float v = ycc[img][3][c];
-                    fa[i][0] = fmaf(we, v, fa[i][0]);  // dx   (edge)
-                    fa[i][1] = fmaf(wp, v, fa[i][1]);  // ddx  (point)
-                    fa[i][2] = fmaf(wg, v, fa[i][2]);  // value (gauss)
-                    ca[i][0] = fmaf(w0, Yv, ca[i][0]);
-                    ca[i][1] = fmaf(w1, ycc[img][1][c], ca[i][1]);
-                    ca[i][2] = fmaf(w2, ycc[img][2][c], ca[i][2]);
-                }
+            for (int i = 0; i < 4; i++) {
+                const int c = xl + i - j + R;
+                const float Yv = ycc[img][0][c];
+                const float v = ycc[img][3][c];
+                fa[i][0] = fmaf(we, v, fa[i][0]);  // dx   (edge)
+                fa[i][1] = fmaf(wp, v, fa[i][1]);  // ddx  (point)
+                fa[i][2] = fmaf(wg, v, fa[i][2]);  // value (gauss)
+                ca[i][0] = fmaf(w0, Yv, ca[i][0]);
+                ca[i][1] = fmaf(w1, ycc[img][1][c], ca[i][1]);
+                ca[i][2] = fmaf(w2, ycc[img][2][c], ca[i][2]);
             }
         }
         const long long p0 = (long long)y * P.w + x0 + xl;
@@ -269,9 +222,9 @@ __device__ __forceinline__ float lab_f(float v) {
 }
 __device__ __forceinline__ float2 lab_f2(float2 v) { return make_float2(lab_f(v.x), lab_f(v.y)); }
 
-// filtered YCxCz -> Hunt-adjusted L*a*b* (shaders/flip/spatial_prefilter.glsl:74-99) of both
+// filtered YCxCz -> the companded XYZ terms of L*a*b* (shaders/flip/spatial_prefilter.glsl:74-96) of both
 // images at once
-__device__ __forceinline__ void ycxcz_to_hunt_lab2(const FlipTaps &T, float2 Y, float2 Cx, float2 Cz, float2 lab[3]) {
+__device__ __forceinline__ void ycxcz_to_lab_terms2(const FlipTaps &T, float2 Y, float2 Cx, float2 Cz, float2 (&c)[3]) {
     const float2 yy = mul2(add2(Y, dup2(16.0f)), dup2(1.0f / 116.0f));
     const float2 cx = mul2(Cx, dup2(1.0f / 500.0f)), cz = mul2(Cz, dup2(1.0f / 200.0f));
     const float2 X = mul2(add2(yy, cx), dup2(T.white[0])), Yw = mul2(yy, dup2(T.white[1]));
@@ -283,18 +236,33 @@ __device__ __forceinline__ void ycxcz_to_hunt_lab2(const FlipTaps &T, float2 Y, 
                               fma2(dup2(T.xyz2rgb[3 * i + 1]), Yw, mul2(dup2(T.xyz2rgb[3 * i + 2]), Z)));
         rgb[i] = make_float2(fminf(fmaxf(v.x, 0.0f), 1.0f), fminf(fmaxf(v.y, 0.0f), 1.0f));
     }
-    float2 c[3];
 #pragma unroll
     for (int i = 0; i < 3; i++)
         c[i] = lab_f2(mul2(fma2(dup2(T.rgb2xyz[3 * i]), rgb[0],
                                 fma2(dup2(T.rgb2xyz[3 * i + 1]), rgb[1], mul2(dup2(T.rgb2xyz[3 * i + 2]), rgb[2]))),
                            dup2(T.inv_white[i])));
-    lab[0] = fma2(dup2(116.0f), c[1], dup2(-16.0f));
-    lab[1] = mul2(dup2(500.0f), sub2(c[0], c[1]));
-    lab[2] = mul2(dup2(200.0f), sub2(c[1], c[2]));
-    const float2 s = mul2(dup2(0.01f), lab[0]);
+}
+
+// The FLIP value from the squared edge and point magnitudes of both images and their companded XYZ terms:
+// Hunt-adjusted L*a*b* (spatial_prefilter.glsl:97-99, with k = 116, -16, 500, 200, 0.01), feature error (feature_detection.glsl:48-53), HyAB
+// colour error (spatial_detection.glsl:67-82) and their combination (combine_error_maps.glsl:28).
+__device__ __forceinline__ float flip_value(float2 g2, float2 p2, const float2 (&c)[3], const float2 (&k)[5], float pcc,
+                                            float dec_lo, float dec_inv_span) {
+    float2 lab[3];
+    lab[0] = fma2(k[0], c[1], k[1]);
+    lab[1] = mul2(k[2], sub2(c[0], c[1]));
+    lab[2] = mul2(k[3], sub2(c[1], c[2]));
+    const float2 s = mul2(k[4], lab[0]);
     lab[1] = mul2(lab[1], s);
     lab[2] = mul2(lab[2], s);
+    const float ed = fabsf(sqrt_nonneg(g2.x) - sqrt_nonneg(g2.y));
+    const float pd = fabsf(sqrt_nonneg(p2.x) - sqrt_nonneg(p2.y));
+    const float def = sqrt_nonneg(0.70710678f * fmaxf(ed, pd));
+    const float d0 = lab[0].x - lab[0].y, d1 = lab[1].x - lab[1].y, d2 = lab[2].x - lab[2].y;
+    const float hy = fabsf(d0) + sqrt_nonneg(fmaf(d1, d1, d2 * d2));
+    const float de = pow_nonneg(hy, 0.7f);
+    const float dec = de < pcc ? dec_lo * de : 0.95f + ((de - pcc) * dec_inv_span) * (1.0f - 0.95f);
+    return pow_nonneg(dec, 1.0f - def);
 }
 
 // Per-pixel FLIP value from the vertically filtered terms of both images, f[q] = {input,
@@ -305,16 +273,10 @@ __device__ __forceinline__ void ycxcz_to_hunt_lab2(const FlipTaps &T, float2 Y, 
 // exactly 0.
 __device__ __forceinline__ float flip_pixel2(const FlipTaps &T, const float2 (&f)[7]) {
     const float2 g2 = fma2(f[0], f[0], mul2(f[1], f[1])), p2 = fma2(f[2], f[2], mul2(f[3], f[3]));
-    float2 lab[3];
-    ycxcz_to_hunt_lab2(T, f[4], f[5], f[6], lab);
-    const float ed = fabsf(sqrt_nonneg(g2.x) - sqrt_nonneg(g2.y));
-    const float pd = fabsf(sqrt_nonneg(p2.x) - sqrt_nonneg(p2.y));
-    const float def = sqrt_nonneg(0.70710678f * fmaxf(ed, pd));
-    const float d0 = lab[0].x - lab[0].y, d1 = lab[1].x - lab[1].y, d2 = lab[2].x - lab[2].y;
-    const float hy = fabsf(d0) + sqrt_nonneg(fmaf(d1, d1, d2 * d2));
-    const float de = pow_nonneg(hy, 0.7f);
-    const float dec = de < T.pcc ? T.dec_lo * de : 0.95f + ((de - T.pcc) * T.dec_inv_span) * (1.0f - 0.95f);
-    return pow_nonneg(dec, 1.0f - def);
+    float2 c[3];
+    ycxcz_to_lab_terms2(T, f[4], f[5], f[6], c);
+    const float2 k[5] = {dup2(116.0f), dup2(-16.0f), dup2(500.0f), dup2(200.0f), dup2(0.01f)};
+    return flip_value(g2, p2, c, k, T.pcc, T.dec_lo, T.dec_inv_span);
 }
 
 // the 7 filtered terms of both images from per-image accumulators
@@ -357,7 +319,6 @@ __device__ __forceinline__ void pool_tile(const FlipArgs &args, const FlipPairDe
     }
 }
 
-template <int RF, int RC>
 __global__ void __launch_bounds__(VT) flip_vpass_kernel(FlipArgs args, const __grid_constant__ FlipTaps T) {
     extern __shared__ float vs[];  // [NPLANE][rows][VT_COLS]
     __shared__ double red[VT / 32];
@@ -367,7 +328,7 @@ __global__ void __launch_bounds__(VT) flip_vpass_kernel(FlipArgs args, const __g
     const FlipPairDev P = args.pairs[pi];
     const int local = gt - P.tile_base;
     const int x0 = (local % P.tiles_x) * VT_COLS, y0 = (local / P.tiles_x) * VT_ROWS;
-    const int rf = RF ? RF : T.rf, rc = RC ? RC : T.rc;
+    const int rf = T.rf, rc = T.rc;
     const int R = max(rf, rc);
     const int rows = VT_ROWS + 2 * R;
     const int n = P.w * P.h;
@@ -437,97 +398,227 @@ __global__ void __launch_bounds__(VT) flip_vpass_kernel(FlipArgs args, const __g
 }
 
 // ---------------------------------------------------------------------------------------------
-// Vertical pass for compile-time radii ("column walkers").  Warp w of a CTA runs role w -- one
-// (image, plane, filter) combination -- down the CTA's 32 columns over CW_BLOCKS blocks of
-// K = 2R+1 rows, keeping the last K rows of its plane in a register window whose slots are fixed
-// at compile time (slot = input row mod K), so each output row costs one coalesced load and the
-// filter's FMAs.  After every block the CTA turns the 14 filtered values of each of its K x 32
-// pixels into FLIP values (flip_pixel) from a shared-memory buffer.
-constexpr int CW_ROLES = 14;         // per image: dx*g, value*edge, ddx*g, value*point, Y*csf0, Cx*csf1, Cz*csf2
-constexpr int CW_T = 32 * CW_ROLES;  // 448 threads
-constexpr int CW_BLOCKS = 10;        // K-row blocks per CTA
-constexpr int CW_GROUP = 2;          // blocks filtered before each pixel phase (2 x 21 x 32 = 3 pixels a thread)
-static_assert(CW_BLOCKS % CW_GROUP == 0, "a CTA's blocks split into whole groups");
+// Both passes in one kernel for radii up to FUSED_MAXR.  A CTA streams down a strip of FW columns, FROWS
+// rows a step, through four phases with a barrier after each:
+//   stage    the rows' pixels (with R columns either side, clamped) of both images, read during the step
+//            before, as (Y, X - Y, Y - Z) of the normalised XYZ: the colour matrices fold the scales of
+//            YCxCz, which are linear, and (Y + 16) / 116 of the shaders is this Y;
+//   rows     each of the six horizontal filters, four neighbouring columns a thread;
+//   columns  a warp a filter and 32 columns: the seven vertical filters as transposed filters, whose
+//            running sums move up one register a row, so that no row is read twice;
+//   pixels   the FLIP value of every pixel whose window is complete.
+// Every value is a float2 {input, reference}, so both images go through the same instructions.  The 12
+// horizontal planes never leave shared memory (200 MB of HBM traffic a 1080p pair otherwise).
+constexpr int FUSED_MAXR = 14;
+constexpr int FW = 64;                 // columns of a strip
+constexpr int FROWS = 14;              // rows of a step: two rounds of pixels, three of row filters
+constexpr int FT_THREADS = 7 * FW;     // a thread a vertical filter and column
+constexpr int HFILT = 6, VFILT = 7;
 
-__host__ __device__ constexpr int cw_rows(int rf, int rc) { return CW_BLOCKS * (2 * (rf > rc ? rf : rc) + 1); }
+// The taps by window position u (row or column y - R + u of output y), zero beyond a filter's own radius,
+// in both halves: horizontal edge, point, g (on Y), luma, red-green and blue-yellow CSF; vertical g on
+// edge, edge on g, g on point, point on g, and the three CSFs.
+struct FusedTaps {
+    float2 h[HFILT][2 * FUSED_MAXR + 1];
+    float2 v[VFILT][2 * FUSED_MAXR + 1];
+    float2 lab[9];   // linear RGB -> (Y, X - Y, Y - Z), normalised, in both halves like all that follow
+    float2 rgb[9];   // (X, Y, Z) normalised -> linear RGB
+    float2 xyz[9];   // linear RGB -> (X, Y, Z), normalised
+    float2 k[5];     // 116, -16, 500, 200, 0.01
+    float lin[256];  // sRGB byte -> linear
+    float pcc, dec_lo, dec_inv_span;
+};
 
-// One block of K output rows: window slot (j + u) % K holds image row y - R + u of output row
-// y = ybase + R + j, weighted by taps[u].  Every role runs this one body (one copy of the unrolled
-// code for all warps); a role whose filter is shorter than K has zero taps at the ends, which leave
-// its sums unchanged bit for bit.
-template <int K>
-__device__ __forceinline__ void cw_block(float (&win)[K], const float (&taps)[K], const float *col, int w, int h,
-                                         int ybase, float *out) {
+// the swizzle of 16-byte units under which every other unit is as good as every unit
+__device__ __forceinline__ int spread(int pair) { return pair ^ ((pair >> 3) & 1); }
+__device__ __forceinline__ int spread2(int i) { return (spread(i >> 1) << 1) | (i & 1); }
+
+template <int R>
+struct FusedSmem {
+    static constexpr int PW = FW + 2 * R;            // staged columns
+    static constexpr int PITCH = (PW + 31) / 32 * 32;  // row pitch: rows start alike for spread()
+    float2 h[FROWS * HFILT * FW];  // [row][filter][column]
+    union {
+        float2 stage[FROWS * 3 * PITCH];  // [row][plane][column]
+        float2 v[FROWS * VFILT * FW];  // [row][filter][column]
+    };
+    float lin[256];
+};
+
+// The vertical filter ROLE of one column over the step's rows.
+template <int R, int ROLE>
+__device__ __forceinline__ void fused_columns(FusedSmem<R> &sm, const FusedTaps &T, int col, float2 (&acc)[2 * R]) {
+    constexpr int K = 2 * R + 1;
+    constexpr int SRC = ROLE == 0 ? 0 : ROLE == 1 ? 2 : ROLE == 2 ? 1 : ROLE == 3 ? 2 : ROLE - 1;
+    const float2 *src = sm.h + SRC * FW + spread2(col);
+    float2 *dst = sm.v + ROLE * FW + col;
+    float2 x = src[0];
+#pragma unroll 2
+    for (int r = 0; r < FROWS; r++) {
+        const float2 next = src[min(r + 1, FROWS - 1) * (HFILT * FW)];
+        dst[r * (VFILT * FW)] = fma2(T.v[ROLE][K - 1], x, acc[0]);
 #pragma unroll
-    for (int j = 0; j < K; j++) {
-        const int y = min(max(ybase + j + K - 1, 0), h - 1);
-        win[(j + K - 1) % K] = __ldg(col + size_t(y) * size_t(w));
-        float acc = 0.f;
-#pragma unroll
-        for (int u = 0; u < K; u++) acc = fmaf(win[(j + u) % K], taps[u], acc);
-        out[j * CW_ROLES * 32] = acc;
+        for (int k = 0; k < K - 2; k++) acc[k] = fma2(T.v[ROLE][K - 2 - k], x, acc[k + 1]);
+        acc[K - 2] = mul2(T.v[ROLE][0], x);
+        x = next;
     }
 }
 
-template <int RF, int RC>
-__global__ void __launch_bounds__(CW_T, 2) flip_vcols_kernel(FlipArgs args, const __grid_constant__ FlipTaps T) {
-    constexpr int R = RF > RC ? RF : RC;
-    constexpr int K = 2 * R + 1;
-    constexpr int SEG = cw_rows(RF, RC);
-    extern __shared__ float cw_buf[];  // [CW_GROUP * K rows][CW_ROLES][32 columns]
-    __shared__ double red[CW_T / 32];
+// Horizontal filter F (and G, of the same plane, unless it is negative) of four neighbouring columns of a row.
+template <int R, int F, int G>
+__device__ __forceinline__ void fused_rows(FusedSmem<R> &sm, const FusedTaps &T, int row, int group) {
+    constexpr int K = 2 * R + 1, PLANE = F < 4 ? 0 : F - 3, N = G < 0 ? 1 : 2;
+    const float4 *src = reinterpret_cast<const float4 *>(sm.stage + (row * 3 + PLANE) * FusedSmem<R>::PITCH);
+    float2 out[N][4];
+#pragma unroll
+    for (int c = 0; c < R + 2; c++) {
+        const float4 two = src[spread(2 * group + c)];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int i = 2 * c + e;  // column 4 group + i of the window
+            const float2 x = e ? make_float2(two.z, two.w) : make_float2(two.x, two.y);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (i - j < 0 || i - j >= K) continue;
+#pragma unroll
+                for (int q = 0; q < N; q++) {
+                    const float2 t = T.h[q ? G : F][i - j];
+                    out[q][j] = i == j ? mul2(t, x) : fma2(t, x, out[q][j]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+        float4 *dst = reinterpret_cast<float4 *>(sm.h + (row * HFILT + (q ? G : F)) * FW);
+        dst[spread(2 * group)] = make_float4(out[q][0].x, out[q][0].y, out[q][1].x, out[q][1].y);
+        dst[spread(2 * group + 1)] = make_float4(out[q][2].x, out[q][2].y, out[q][3].x, out[q][3].y);
+    }
+}
+
+// FLIP value of one pixel from its seven vertically filtered terms.
+__device__ __forceinline__ float fused_pixel(const FusedTaps &T, const float2 (&f)[VFILT]) {
+    const float2 g2 = fma2(f[0], f[0], mul2(f[1], f[1])), p2 = fma2(f[2], f[2], mul2(f[3], f[3]));
+    const float2 X = add2(f[4], f[5]), Z = sub2(f[4], f[6]);
+    float2 rgb[3], c[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const float2 v = fma2(T.rgb[3 * i], X, fma2(T.rgb[3 * i + 1], f[4], mul2(T.rgb[3 * i + 2], Z)));
+        rgb[i] = make_float2(__saturatef(v.x), __saturatef(v.y));
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+        c[i] = lab_f2(fma2(T.xyz[3 * i], rgb[0], fma2(T.xyz[3 * i + 1], rgb[1], mul2(T.xyz[3 * i + 2], rgb[2]))));
+    return flip_value(g2, p2, c, T.k, T.pcc, T.dec_lo, T.dec_inv_span);
+}
+
+// Bound by the FMA pipe (54% busy at 67 ppd, of 830 instructions a pixel pair 290 are taps) with 28 warps an
+// SM and four barriers a step.  Four 1080p pairs at 38 / 52 / 67 ppd: 247 / 305 / 382 us; the two passes
+// through HBM planes took 972 us with runtime radii and 421 / 392 us with radii built in (7, 8 and 9, 10).
+// Shared memory holds two CTAs, whose 72 registers carry the running sums (a few spill between phases);
+// beyond radius 11 one CTA with 128 registers is left.
+template <int R>
+__global__ void __launch_bounds__(FT_THREADS, R <= 11 ? 2 : 1) flip_kernel(FlipArgs args, const __grid_constant__ FusedTaps T) {
+    using Sm = FusedSmem<R>;
+    constexpr int PW = Sm::PW, COLS = (PW + 15) / 16 * 16, GROUPS = FT_THREADS / COLS;  // rows staged at once
+    constexpr int PER_T = (FROWS + GROUPS - 1) / GROUPS;
+    extern __shared__ __align__(16) unsigned char flip_smem[];
+    Sm &sm = *reinterpret_cast<Sm *>(flip_smem);
+    __shared__ double red[FT_THREADS / 32];
     __shared__ int is_last;
     const int gt = blockIdx.x;
     const int pi = find_tile(args.pairs, args.npairs, gt);
     const FlipPairDev P = args.pairs[pi];
     const int local = gt - P.tile_base;
-    const int x0 = (local % P.tiles_x) * 32, y0 = (local / P.tiles_x) * SEG;
-    const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
-    const int f = role % 7, m = role / 7;
-    // plane of each role within the image's six: dx, ddx, value, Y, Cx, Cz
-    const int pl = m * 6 + (f == 0 ? 0 : f == 1 ? 2 : f == 2 ? 1 : f == 3 ? 2 : f - 1);
-    const size_t n = size_t(P.w) * size_t(P.h);
-    const float *col = args.planes + P.plane_off + size_t(pl) * n + min(x0 + lane, P.w - 1);
-    // this role's taps: image row y - k weighs tap k + radius; feature roles use g, edge, g, point
-    const float *tap_src = f < 4 ? T.feat[f == 1 ? 1 : f == 3 ? 2 : 0] : T.csf[f - 4];
-    const int rad = f < 4 ? RF : RC;
-    float win[K];
+    const int x0 = (local % P.tiles_x) * FW, y0 = (local / P.tiles_x) * args.strip;
+    const int y1 = min(y0 + args.strip, P.h);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int i = tid; i < 256; i += FT_THREADS) sm.lin[i] = T.lin[i];
+
+    // this thread's share of the staging: one column of every GROUPS-th row
+    const int grp = tid / COLS, sc = tid - grp * COLS;
+    const bool stages = grp < GROUPS && sc < PW;
+    const int sx = min(max(x0 - R + sc, 0), P.w - 1);
+    uint32_t ra[PER_T], rb[PER_T];
+    auto load = [&](int s) {
+        if (!stages) return;
 #pragma unroll
-    for (int t = 0; t < K - 1; t++) win[t] = __ldg(col + size_t(min(max(y0 - R + t, 0), P.h - 1)) * size_t(P.w));
-    float *out = cw_buf + role * 32 + lane;
-    double dsum = 0.0;
-    for (int b = 0; b < CW_BLOCKS; b += CW_GROUP) {
-        const int yg = y0 + b * K;
-        if (yg >= P.h) break;  // uniform over the CTA
-        for (int bb = 0; bb < CW_GROUP; bb++) {
-            const int yb = yg + bb * K;
-            if (yb >= P.h) break;  // uniform; rows past the image are skipped by the pixel phase
-            float taps[K];  // reloaded per block so they are not live across the pixel phase
+        for (int k = 0; k < PER_T; k++) {
+            const int row = grp + k * GROUPS;
+            if (row >= FROWS) continue;
+            const long long at = min(max(y0 - R + s * FROWS + row, 0), P.h - 1) * P.pitch + 4LL * sx;
+            ra[k] = __ldg(reinterpret_cast<const uint32_t *>(P.a + at));
+            rb[k] = __ldg(reinterpret_cast<const uint32_t *>(P.b + at));
+        }
+    };
+    float2 acc[2 * R];
 #pragma unroll
-            for (int u = 0; u < K; u++) {
-                const int k = R - u;
-                taps[u] = (k >= -rad && k <= rad) ? tap_src[k + rad] : 0.f;
+    for (int k = 0; k < 2 * R; k++) acc[k] = make_float2(0.f, 0.f);
+    long long sum = 0;   // of the pixels' values, in units of 2^-28
+    double other = 0.0;  // values that are no such numbers
+    const int steps = (y1 - y0 + 2 * R + FROWS - 1) / FROWS;
+    load(0);
+    __syncthreads();  // the sRGB table
+#pragma unroll 1
+    for (int s = 0; s < steps; s++) {
+        if (stages) {
+            float2 *dst = sm.stage + spread2(sc);
+#pragma unroll
+            for (int k = 0; k < PER_T; k++) {
+                const int row = grp + k * GROUPS;
+                if (row >= FROWS) continue;
+                const float2 r = make_float2(sm.lin[ra[k] & 0xffu], sm.lin[rb[k] & 0xffu]);
+                const float2 g = make_float2(sm.lin[(ra[k] >> 8) & 0xffu], sm.lin[(rb[k] >> 8) & 0xffu]);
+                const float2 b = make_float2(sm.lin[(ra[k] >> 16) & 0xffu], sm.lin[(rb[k] >> 16) & 0xffu]);
+#pragma unroll
+                for (int p = 0; p < 3; p++)
+                    dst[(row * 3 + p) * Sm::PITCH] =
+                        fma2(T.lab[3 * p], r, fma2(T.lab[3 * p + 1], g, mul2(T.lab[3 * p + 2], b)));
             }
-            cw_block<K>(win, taps, col, P.w, P.h, yb - R, out + bb * K * CW_ROLES * 32);
         }
         __syncthreads();
-        for (int p = threadIdx.x; p < CW_GROUP * K * 32; p += CW_T) {
-            const int j = p >> 5, c = p & 31;
-            const int y = yg + j, x = x0 + c;
-            if (y >= P.h || x >= P.w) continue;
-            float v[2][7];
-            const float *px = cw_buf + j * CW_ROLES * 32 + c;
+        if (s + 1 < steps) load(s + 1);
+        {
+            const int row = (warp % 7) * 2 + (lane >> 4), group = lane & 15;
+            if (warp < 7) {  // half of the filters here, half there
+                fused_rows<R, 0, 2>(sm, T, row, group);
+                fused_rows<R, 4, -1>(sm, T, row, group);
+            } else {
+                fused_rows<R, 1, 3>(sm, T, row, group);
+                fused_rows<R, 5, -1>(sm, T, row, group);
+            }
+        }
+        __syncthreads();
+        {
+            const int col = (warp & 1) * 32 + lane;
+            switch (warp >> 1) {
+                case 0: fused_columns<R, 0>(sm, T, col, acc); break;
+                case 1: fused_columns<R, 1>(sm, T, col, acc); break;
+                case 2: fused_columns<R, 2>(sm, T, col, acc); break;
+                case 3: fused_columns<R, 3>(sm, T, col, acc); break;
+                case 4: fused_columns<R, 4>(sm, T, col, acc); break;
+                case 5: fused_columns<R, 5>(sm, T, col, acc); break;
+                default: fused_columns<R, 6>(sm, T, col, acc); break;
+            }
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int p = tid; p < FROWS * FW; p += FT_THREADS) {
+            const int row = p / FW, c = p - row * FW;
+            const int y = y0 - 2 * R + s * FROWS + row, x = x0 + c;
+            if (y < y0 || y >= y1 || x >= P.w) continue;
+            float2 f[VFILT];
 #pragma unroll
-            for (int mm = 0; mm < 2; mm++)
-#pragma unroll
-                for (int q = 0; q < 7; q++) v[mm][q] = px[(mm * 7 + q) * 32];
-            const float val = flip_pixel(T, v);
+            for (int q = 0; q < VFILT; q++) f[q] = sm.v[(row * VFILT + q) * FW + c];
+            const float val = fused_pixel(T, f);
             if (P.map) P.map[size_t(y) * size_t(P.w) + x] = val;
-            dsum += double(val);
+            if (fabsf(val) < 4.0f) sum += __float2int_rn(val * 268435456.0f);
+            else other += val;
         }
-        __syncthreads();
+        __syncthreads();  // the filtered values are read before the next rows are staged
     }
-    pool_tile<CW_T>(args, P, pi, gt, dsum, red, is_last);
+    // Sums of these are exact in FP64 (up to 2^25 pixels), so the cut into strips does not matter.
+    pool_tile<FT_THREADS>(args, P, pi, gt, double(sum) * (1.0 / 268435456.0) + other, red, is_last);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -634,14 +725,95 @@ void check_params(const iqm_flip_params &p) {
                 "FLIP monitor parameters must be positive");
 }
 
+constexpr int FUSED_MINR = 3;  // smaller radii run as 3, with zero taps
+
+FusedTaps fused_taps(const FlipTaps &T, int R) {
+    FusedTaps F{};
+    for (int u = 0; u <= 2 * R; u++) {
+        const int j = R - u;  // output x takes tap j of the pixel at x - j
+        auto at = [&](const float *t, int rad) { return j >= -rad && j <= rad ? make_float2(t[j + rad], t[j + rad]) : make_float2(0.f, 0.f); };
+        const float2 g = at(T.feat[0], T.rf), edge = at(T.feat[1], T.rf), point = at(T.feat[2], T.rf);
+        F.h[0][u] = edge;
+        F.h[1][u] = point;
+        F.h[2][u] = g;
+        F.v[0][u] = F.v[2][u] = g;
+        F.v[1][u] = edge;
+        F.v[3][u] = point;
+        for (int c = 0; c < 3; c++) F.h[3 + c][u] = F.v[4 + c][u] = at(T.csf[c], T.rc);
+    }
+    auto both = [](double v) { return make_float2(float(v), float(v)); };
+    double xyz[9];
+    for (int i = 0; i < 3; i++)
+        for (int k = 0; k < 3; k++) {
+            xyz[3 * i + k] = double(T.rgb2xyz[3 * i + k]) / double(T.white[i]);
+            F.xyz[3 * i + k] = both(xyz[3 * i + k]);
+            F.rgb[3 * i + k] = both(double(T.xyz2rgb[3 * i + k]) * double(T.white[k]));
+        }
+    for (int k = 0; k < 3; k++) {
+        F.lab[k] = both(xyz[3 + k]);
+        F.lab[3 + k] = both(xyz[k] - xyz[3 + k]);
+        F.lab[6 + k] = both(xyz[3 + k] - xyz[6 + k]);
+    }
+    const double k[5] = {116.0, -16.0, 500.0, 200.0, 0.01};
+    for (int i = 0; i < 5; i++) F.k[i] = both(k[i]);
+    for (int i = 0; i < 256; i++) F.lin[i] = T.lin[i];
+    F.pcc = T.pcc;
+    F.dec_lo = T.dec_lo;
+    F.dec_inv_span = T.dec_inv_span;
+    return F;
+}
+
+// Output rows of a tile, the same for all pairs of a launch: whole steps of FROWS rows less the window's
+// 2 R, of the least estimated time (a tile's steps and a step's worth of set-up, times the rounds of two
+// CTAs per SM).  No value depends on the choice.
+int strip_rows(const std::vector<iqm_pair> &pairs, int R) {
+    int best = 0;
+    double best_cost = 0.0;
+    for (int steps = 12; FROWS * steps > 2 * R; steps--) {
+        const int s = FROWS * steps - 2 * R;
+        double tiles = 0.0;
+        for (const iqm_pair &p : pairs) tiles += double(iqm::ceil_div(p.w, FW)) * iqm::ceil_div(p.h, s);
+        const double cost = (steps + 1) * std::max(1.0, tiles / (2 * 148));
+        if (!best || cost < best_cost) {
+            best = s;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+void launch_fused(const FlipArgs &a, const FlipTaps &T, int R, int tiles, cudaStream_t st) {
+    const FusedTaps F = fused_taps(T, R);
+    auto go = [&](auto r) {
+        constexpr int RR = decltype(r)::value;
+        const size_t smem = sizeof(FusedSmem<RR>);
+        IQM_CHECK_CUDA(cudaFuncSetAttribute((const void *)flip_kernel<RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        flip_kernel<RR><<<tiles, FT_THREADS, smem, st>>>(a, F);
+    };
+    switch (R) {
+        case 3: go(std::integral_constant<int, 3>{}); break;
+        case 4: go(std::integral_constant<int, 4>{}); break;
+        case 5: go(std::integral_constant<int, 5>{}); break;
+        case 6: go(std::integral_constant<int, 6>{}); break;
+        case 7: go(std::integral_constant<int, 7>{}); break;
+        case 8: go(std::integral_constant<int, 8>{}); break;
+        case 9: go(std::integral_constant<int, 9>{}); break;
+        case 10: go(std::integral_constant<int, 10>{}); break;
+        case 11: go(std::integral_constant<int, 11>{}); break;
+        case 12: go(std::integral_constant<int, 12>{}); break;
+        case 13: go(std::integral_constant<int, 13>{}); break;
+        default: go(std::integral_constant<int, 14>{}); break;
+    }
+}
+
 void flip_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, const iqm_flip_params &params,
                   const std::vector<float *> &maps, double *d_scores) {
     FlipTaps T{};
     make_taps(ppd_of(params), T);
     const int n = int(pairs.size());
-    // the two viewing set-ups in common use get kernels with their radii built in
-    const int fixed = (T.rf == 7 && T.rc == 8) ? 1 : (T.rf == 9 && T.rc == 10) ? 2 : 0;
-    const int tile_rows = fixed == 1 ? cw_rows(7, 8) : fixed == 2 ? cw_rows(9, 10) : VT_ROWS;
+    const int R = std::max(T.rf, T.rc);
+    const bool fused = R <= FUSED_MAXR;
+    const int strip = fused ? strip_rows(pairs, std::max(R, FUSED_MINR)) : VT_ROWS;
     std::vector<FlipPairDev> hd(n);
     long long segs = 0, plane_floats = 0;
     int tiles = 0;
@@ -654,15 +826,15 @@ void flip_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, const iqm_fl
         d.pitch = (long long)q.row_bytes;
         d.w = q.w;
         d.h = q.h;
-        d.tiles_x = int(iqm::ceil_div(q.w, VT_COLS));
-        d.ntiles = d.tiles_x * int(iqm::ceil_div(q.h, tile_rows));
+        d.tiles_x = int(iqm::ceil_div(q.w, fused ? FW : VT_COLS));
+        d.ntiles = d.tiles_x * int(iqm::ceil_div(q.h, strip));
         d.tile_base = tiles;
         d.vec_ok = 0;
         d.plane_off = plane_floats;
         d.seg_base = segs;
         tiles += d.ntiles;
         segs += (long long)iqm::ceil_div(q.w, HSEG) * iqm::ceil_div(q.h, HROWS);
-        plane_floats += (long long)NPLANE * q.w * q.h;
+        if (!fused) plane_floats += (long long)NPLANE * q.w * q.h;
     }
     IQM_REQUIRE(segs < (1LL << 31) && tiles < (1 << 30), "batch too large");
     auto *d_desc = static_cast<FlipPairDev *>(iqm::upload_bytes(ctx, ctx->desc, hd.data(), sizeof(FlipPairDev) * n));
@@ -680,35 +852,19 @@ void flip_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, const iqm_fl
     a.total_segs = segs;
     IQM_CHECK_CUDA(cudaMemsetAsync(a.counters, 0, sizeof(unsigned) * n, ctx->stream));
     iqm::timing_mark(ctx, nullptr);
-    const int R = std::max(T.rf, T.rc);
-    const size_t smem = sizeof(float) * NPLANE * (VT_ROWS + 2 * R) * VT_COLS;
-    // dynamic shared memory of the column walkers: CW_GROUP blocks of K rows x 14 roles x 32 columns
-    auto cw_smem = [](int rf, int rc) { return sizeof(float) * CW_GROUP * (2 * std::max(rf, rc) + 1) * CW_ROLES * 32; };
-    if (fixed == 1) {  // default monitor, 52.1 ppd
-        flip_hpass_kernel<7, 8><<<unsigned(segs), HT, 0, ctx->stream>>>(a, T);
-        iqm::check_launch(ctx, "flip_hpass_kernel");
-        const size_t sm = cw_smem(7, 8);
-        IQM_CHECK_CUDA(cudaFuncSetAttribute((const void *)flip_vcols_kernel<7, 8>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-        flip_vcols_kernel<7, 8><<<tiles, CW_T, sm, ctx->stream>>>(a, T);
-        iqm::check_launch(ctx, "flip_vcols_kernel");
-    } else if (fixed == 2) {  // 67 ppd
-        flip_hpass_kernel<9, 10><<<unsigned(segs), HT, 0, ctx->stream>>>(a, T);
-        iqm::check_launch(ctx, "flip_hpass_kernel");
-        const size_t sm = cw_smem(9, 10);
-        IQM_CHECK_CUDA(cudaFuncSetAttribute((const void *)flip_vcols_kernel<9, 10>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-        flip_vcols_kernel<9, 10><<<tiles, CW_T, sm, ctx->stream>>>(a, T);
-        iqm::check_launch(ctx, "flip_vcols_kernel");
-    } else {
-        flip_hpass_kernel<0, 0><<<unsigned(segs), HT, 0, ctx->stream>>>(a, T);
-        iqm::check_launch(ctx, "flip_hpass_kernel");
-        if (smem > 48 * 1024)
-            IQM_CHECK_CUDA(cudaFuncSetAttribute((const void *)flip_vpass_kernel<0, 0>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        flip_vpass_kernel<0, 0><<<tiles, VT, smem, ctx->stream>>>(a, T);
-        iqm::check_launch(ctx, "flip_vpass_kernel");
+    if (fused) {
+        a.strip = strip;
+        launch_fused(a, T, std::max(R, FUSED_MINR), tiles, ctx->stream);
+        iqm::check_launch(ctx, "flip_kernel");
+        return;
     }
+    const size_t smem = sizeof(float) * NPLANE * (VT_ROWS + 2 * R) * VT_COLS;
+    flip_hpass_kernel<<<unsigned(segs), HT, 0, ctx->stream>>>(a, T);
+    iqm::check_launch(ctx, "flip_hpass_kernel");
+    if (smem > 48 * 1024)
+        IQM_CHECK_CUDA(cudaFuncSetAttribute((const void *)flip_vpass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    flip_vpass_kernel<<<tiles, VT, smem, ctx->stream>>>(a, T);
+    iqm::check_launch(ctx, "flip_vpass_kernel");
 }
 
 }  // namespace
