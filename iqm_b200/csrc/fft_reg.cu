@@ -61,6 +61,7 @@ RegStep make_step(int radix, int items, int d0, int hi, int lo, int stride) {
     s.items = items;
     s.d0 = d0;
     s.inv_d0 = 1.0f / float(d0);
+    s.inv_items = 1.0f / float(items);
     s.hi = hi;
     s.lo = lo;
     s.stride = stride;
@@ -106,7 +107,7 @@ RegFft build(int n, bool blue, int p1, int p2, int p3) {
         if (blue) add(axis1, false);
     }
     F.nsteps = k;
-    F.inv_items_last = 1.0f / float(F.st[k - 1].items);
+    F.inv_items_last = F.st[k - 1].inv_items;
     return F;
 }
 

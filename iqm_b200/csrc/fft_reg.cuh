@@ -37,6 +37,7 @@ struct RegStep {
     int hi, lo;
     int stride;   // between the points of a line
     int tw;       // offset of the step's twiddles in RegFft::tw (-1: none)
+    float inv_items;
 };
 
 struct RegFft {
@@ -94,7 +95,7 @@ struct ColLayout {
     __device__ __forceinline__ int lc() const { return LC >= 0 ? LC : lc_; }
     __device__ __forceinline__ int first() const { return threadIdx.x; }
     __device__ __forceinline__ int total(int items) const { return items << lc(); }
-    __device__ __forceinline__ void split(int w, int, int &seq, int &i) const {
+    __device__ __forceinline__ void split(int w, const RegStep &, int &seq, int &i) const {
         seq = w & ((1 << lc()) - 1);
         i = w >> lc();
     }
@@ -108,9 +109,9 @@ struct RowLayout {
     int threads;
     __device__ __forceinline__ int first() const { return threadIdx.x; }
     __device__ __forceinline__ int total(int items) const { return items * count; }
-    __device__ __forceinline__ void split(int w, int items, int &seq, int &i) const {
-        seq = div_by(w, 1.0f / float(items));
-        i = w - seq * items;
+    __device__ __forceinline__ void split(int w, const RegStep &S, int &seq, int &i) const {
+        seq = div_by(w, S.inv_items);
+        i = w - seq * S.items;
     }
     __device__ __forceinline__ bool live(int) const { return true; }
     __device__ __forceinline__ int addr(int seq, int a) const { return seq * size + a; }
@@ -131,6 +132,14 @@ __device__ __forceinline__ void twiddle_line(float2 *v, const RegFft &F, const R
     for (int r = R0; r < P; r++) v[r] = cmul(v[r], __ldg(run_at(tw, d, r)));
 }
 
+// Points of line i that are inputs or outputs of a Bluestein transform, i + r items < n: fewer than half the
+// line and one, as n <= (m + 1) / 2, so the rest of the line is left out at compile time.
+template <int P>
+constexpr int kHalf = (P + 2) / 2;
+__device__ __forceinline__ int live_points(const RegFft &F, const RegStep &S, int i) {
+    return div_by(F.n - i + S.items - 1, S.inv_items);
+}
+
 // First step: ld(seq, i, items)(r), element i + r items of a sequence -> lines -> shared memory.
 template <int P, bool BLUE, class Lay, class Ld>
 __device__ __forceinline__ void reg_first(const RegFft &F, const Lay &lay, float2 *sm, Ld &ld) {
@@ -138,21 +147,18 @@ __device__ __forceinline__ void reg_first(const RegFft &F, const Lay &lay, float
     const int total = lay.total(S.items);
     for (int w = lay.first(); w < total; w += lay.threads) {
         int seq, i;
-        lay.split(w, S.items, seq, i);
+        lay.split(w, S, seq, i);
         if (!lay.live(seq)) continue;
         auto src = ld(seq, i, S.items);
         float2 v[P];
         if constexpr (BLUE) {
+            const int live = live_points(F, S, i);
 #pragma unroll
-            for (int r = 0; r < P; r++) {
-                const int k = i + r * S.items;
-                v[r] = k < F.n ? src(r) : make_float2(0.f, 0.f);
-            }
+            for (int r = 0; r < P; r++) v[r] = r < kHalf<P> && r < live ? src(r) : make_float2(0.f, 0.f);
+            const float2 *chirp = F.chirp + i;
 #pragma unroll
-            for (int r = 0; r < P; r++) {
-                const int k = i + r * S.items;
-                if (k < F.n) v[r] = cmul(v[r], __ldg(run_at(F.chirp + i, 8u * S.items, r)));
-            }
+            for (int r = 0; r < kHalf<P>; r++)
+                if (r < live) v[r] = cmul(v[r], __ldg(run_at(chirp, 8u * S.items, r)));
         } else {
 #pragma unroll
             for (int r = 0; r < P; r++) v[r] = src(r);
@@ -174,7 +180,7 @@ __device__ __forceinline__ void reg_middle(const RegFft &F, const RegStep &S, co
     const int total = lay.total(S.items);
     for (int w = lay.first(); w < total; w += lay.threads) {
         int seq, i;
-        lay.split(w, S.items, seq, i);
+        lay.split(w, S, seq, i);
         if (!lay.live(seq)) continue;
         const unsigned p = smem_addr(sm) + 8u * lay.addr(seq, line_base(S, i)), d = 8u * lay.stride(UNIT ? 1 : S.stride);
         float2 v[P];
@@ -201,7 +207,7 @@ __device__ __forceinline__ void reg_last(const RegFft &F, const RegStep &S, cons
     const int total = lay.total(S.items);
     for (int w = lay.first(); w < total; w += lay.threads) {
         int seq, i;
-        lay.split(w, S.items, seq, i);
+        lay.split(w, S, seq, i);
         if (!lay.live(seq)) continue;
         const unsigned p = smem_addr(sm) + 8u * lay.addr(seq, line_base(S, i)), d = 8u * lay.stride(UNIT ? 1 : S.stride);
         float2 v[P];
@@ -209,13 +215,15 @@ __device__ __forceinline__ void reg_last(const RegFft &F, const RegStep &S, cons
         for (int r = 0; r < P; r++) v[r] = lds2(p + r * d);
         dft_reg<P>(v);
         auto dst = st(seq, i, S.items);
+        if constexpr (BLUE) {
+            const int live = live_points(F, S, i);
+            const float2 *chirp = F.chirp + i;
 #pragma unroll
-        for (int r = 0; r < P; r++) {
-            if constexpr (BLUE) {
-                if (i + r * S.items < F.n) dst(r, p + r * d, cmul(make_float2(v[r].y, v[r].x), __ldg(run_at(F.chirp + i, 8u * S.items, r))));
-            } else {
-                dst(r, p + r * d, v[r]);
-            }
+            for (int r = 0; r < kHalf<P>; r++)
+                if (r < live) dst(r, p + r * d, cmul(make_float2(v[r].y, v[r].x), __ldg(run_at(chirp, 8u * S.items, r))));
+        } else {
+#pragma unroll
+            for (int r = 0; r < P; r++) dst(r, p + r * d, v[r]);
         }
     }
 }
