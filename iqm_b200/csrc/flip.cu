@@ -837,21 +837,18 @@ void flip_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, const iqm_fl
         if (!fused) plane_floats += (long long)NPLANE * q.w * q.h;
     }
     IQM_REQUIRE(segs < (1LL << 31) && tiles < (1 << 30), "batch too large");
-    auto *d_desc = static_cast<FlipPairDev *>(iqm::upload_bytes(ctx, ctx->desc, hd.data(), sizeof(FlipPairDev) * n));
-    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t pb = al(sizeof(float) * size_t(plane_floats)), qb = al(sizeof(double) * tiles),
-                 cb = al(sizeof(unsigned) * n);
-    auto *base = static_cast<uint8_t *>(ctx->scratch.get(pb + qb + cb, ctx->stream));
+    unsigned *counters = nullptr;
+    auto *d_desc = static_cast<FlipPairDev *>(iqm::upload_with_counters(ctx, hd.data(), sizeof(FlipPairDev) * n, n, counters));
+    const size_t pb = (sizeof(float) * size_t(plane_floats) + 255) & ~size_t(255);
+    auto *base = static_cast<uint8_t *>(ctx->scratch.get(pb + sizeof(double) * tiles, ctx->stream));
     FlipArgs a{};
     a.pairs = d_desc;
     a.npairs = n;
     a.planes = reinterpret_cast<float *>(base);
     a.partials = reinterpret_cast<double *>(base + pb);
-    a.counters = reinterpret_cast<unsigned *>(base + pb + qb);
+    a.counters = counters;
     a.scores = d_scores;
     a.total_segs = segs;
-    IQM_CHECK_CUDA(cudaMemsetAsync(a.counters, 0, sizeof(unsigned) * n, ctx->stream));
-    iqm::timing_mark(ctx, nullptr);
     if (fused) {
         a.strip = strip;
         launch_fused(a, T, std::max(R, FUSED_MINR), tiles, ctx->stream);

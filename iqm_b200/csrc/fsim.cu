@@ -719,6 +719,7 @@ __global__ void __launch_bounds__(1024, 2) fsim_noise_kernel(FsimGroup g) {
     const int pi = blockIdx.y;
     const int o = q & 3;
     const float *v = g.eo0 + (size_t(pi) * 8 + q) * g.n;
+    iqm::wait_for_previous();
     const float med = iqm::block_select_kth(v, g.n, g.n / 2, hist, stage, NOISE_STAGE);
     if (threadIdx.x == 0) {
         const double mean = -double(med) / log(0.5);
@@ -780,6 +781,7 @@ template <int PX>
 __global__ void __launch_bounds__(FT) fsim_final_kernel(FsimGroup g) {
     __shared__ double red[3][FT / 32];
     __shared__ int is_last;
+    iqm::wait_for_previous();
     const int pi = blockIdx.y;
     const int p = (blockIdx.x * FT + threadIdx.x) * PX;
     const int n = g.n;
@@ -1154,7 +1156,7 @@ iqm::FsimPlan *get_plan(iqm_ctx *ctx, int w2, int h2) {
 }
 
 struct Layout {
-    size_t yiq, spec, spec2, T, planes, thr, partials, counters, total;
+    size_t yiq, spec, spec2, T, planes, thr, partials, total;
 };
 
 // G pairs of the group; chunk pairs' worth of inverse-pass intermediates.
@@ -1171,7 +1173,6 @@ Layout layout_for(int G, int chunk, int n, int tiles, int nbuf, int tiled) {
     L.planes = off; off += al(sizeof(float) * size_t(G) * 24 * n);
     L.thr = off; off += al(sizeof(float) * size_t(G) * 8);
     L.partials = off; off += al(sizeof(double) * size_t(G) * tiles * 3);
-    L.counters = off; off += al(sizeof(unsigned) * size_t(G));
     L.total = off;
     return L;
 }
@@ -1216,8 +1217,9 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
     ordered.reserve(n_pairs);
     for (auto &kv : groups)
         for (int i : kv.second) ordered.push_back(hd[i]);
+    unsigned *counters = nullptr;
     auto *d_desc = static_cast<FsimPairDev *>(
-        iqm::upload_bytes(ctx, ctx->desc, ordered.data(), sizeof(FsimPairDev) * n_pairs));
+        iqm::upload_with_counters(ctx, ordered.data(), sizeof(FsimPairDev) * n_pairs, n_pairs, counters));
     // per-size tables first (building one waits for the context stream)
     struct GroupRun {
         int w2, h2, G, first, slot, F_uniform, chunk;
@@ -1322,14 +1324,13 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
         g.eo0 = g.energy + size_t(G) * 8 * n;
         g.thr = reinterpret_cast<float *>(base + Lc.thr);
         g.partials = reinterpret_cast<double *>(base + Lc.partials);
-        g.counters = reinterpret_cast<unsigned *>(base + Lc.counters);
+        g.counters = counters + r.first;
         g.tiles = tiles;
+        g.early = !r.overlap;
         g.scores = d_scores;
         g.filters = P->filters;
         g.consts = P->consts;
         g.energy_mode = energy_mode;
-        IQM_CHECK_CUDA(cudaMemsetAsync(g.counters, 0, sizeof(unsigned) * G, st));
-        iqm::timing_mark(ctx, nullptr);
         launch_ingest(g, r.F_uniform, tiles, st);
         iqm::check_launch(ctx, "fsim_ingest_kernel");
         if (reg) {
@@ -1379,12 +1380,12 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
             IQM_CHECK_CUDA(cudaEventRecord(ctx->side_events[j * S + r.slot], cstream[j]));
             IQM_CHECK_CUDA(cudaStreamWaitEvent(st, ctx->side_events[j * S + r.slot], 0));
         }
-        fsim_noise_kernel<<<dim3(8, G), 1024, 0, st>>>(g);
+        iqm::launch_after(fsim_noise_kernel, dim3(8, G), 1024, 0, 0, g.early, st, g);
         iqm::check_launch(ctx, "fsim_noise_kernel");
         if (w2 % 4 == 0)
-            fsim_final_kernel<4><<<dim3(int(iqm::ceil_div(n, 4 * FT)), G), FT, 0, st>>>(g);
+            iqm::launch_after(fsim_final_kernel<4>, dim3(int(iqm::ceil_div(n, 4 * FT)), G), FT, 0, 0, g.early, st, g);
         else
-            fsim_final_kernel<1><<<dim3(tiles, G), FT, 0, st>>>(g);
+            iqm::launch_after(fsim_final_kernel<1>, dim3(tiles, G), FT, 0, 0, g.early, st, g);
         iqm::check_launch(ctx, "fsim_final_kernel");
     }
     if (S > 1) {

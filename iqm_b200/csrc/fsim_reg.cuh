@@ -40,19 +40,11 @@ int resident_ctas(const void *fn, int threads, size_t smem, bool carveout = true
 // Launches a transform kernel with just the shared memory its resident CTAs use, so that the rest of the
 // SM's array serves as L1 for the twiddles and for the spectrum that every scale reads again.
 template <class... Params, class... Args>
-inline void launch_transform(void (*fn)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+inline void launch_transform(void (*fn)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, const FsimGroup &g,
+                             Args... args) {
     const int ctas = resident_ctas((const void *)fn, threads, smem, false);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-    attr.val.sharedMemCarveout = unsigned(std::min<size_t>(100, (ctas * (smem + 2048) * 100 + 228 * 1024 - 1) / (228 * 1024)));
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    IQM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, fn, Params(args)...));
+    const size_t share = (ctas * (smem + 2048) * 100 + 228 * 1024 - 1) / (228 * 1024);
+    launch_after(fn, grid, threads, smem, int(std::min<size_t>(100, share)), g.early, st, g, args...);
 }
 
 template <class F>

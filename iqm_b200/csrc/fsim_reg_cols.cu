@@ -32,8 +32,9 @@ fsim_inv_cols_reg(FsimGroup g, const __grid_constant__ RegFft F, int lc_) {
     const float2 *S = g.spec2 + (size_t(g.pair0) * 2 + plane) * g.tiled + size_t(blockIdx.x) * g.tile;
     const float *H = g.filters + size_t(o * 4) * g.tiled + size_t(blockIdx.x) * g.tile;
     const unsigned s_tile = smem_addr(sm) + 8u * (((F.size << lc) + 1) & ~1), h_tile = s_tile + 8u * g.tile;
+    copy_run(h_tile, H, 4 * g.tile);  // the plan's, not the previous kernel's
+    wait_for_previous();
     copy_run(s_tile, S, 8 * g.tile);
-    copy_run(h_tile, H, 4 * g.tile);
     copy_commit();
     const ColLayout<LC> lay{lc, min(1 << lc, w2 - x0), int(blockDim.x)};
     for (int s = 0; s < 4; s++) {

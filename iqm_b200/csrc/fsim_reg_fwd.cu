@@ -10,6 +10,7 @@ template <int KIND>
 __global__ void __launch_bounds__(reg_most_threads(KIND), reg_min_ctas(KIND))
 fsim_fwd_rows_reg(FsimGroup g, const __grid_constant__ RegFft F, int rows) {
     extern __shared__ __align__(16) float2 sm[];
+    wait_for_previous();
     const int y0 = blockIdx.x * rows, pair = blockIdx.y;
     const float *Y1 = g.yiq + (size_t(pair * 2) * 3 + 2) * g.n + size_t(y0) * g.w2;
     const float *Y2 = Y1 + size_t(3) * g.n;
@@ -34,6 +35,7 @@ template <int KIND>
 __global__ void __launch_bounds__(reg_most_threads(KIND), reg_min_ctas(KIND))
 fsim_fwd_cols_reg(FsimGroup g, const __grid_constant__ RegFft F, int lc) {
     extern __shared__ __align__(16) float2 sm[];
+    wait_for_previous();
     const int half = 1 << (lc - 1);          // slots [0, half): columns x0 + c; the rest: columns -(x0 + c)
     const int x0 = blockIdx.x * half, pair = blockIdx.y;
     const int w2 = g.w2, h2 = g.h2;

@@ -11,6 +11,7 @@ template <int KIND>
 __global__ void __launch_bounds__(reg_most_threads(KIND), reg_min_ctas(KIND))
 fsim_inv_rows_reg(FsimGroup g, const __grid_constant__ RegFft F, int rows, double *rowsums) {
     extern __shared__ __align__(16) float2 sm[];
+    wait_for_previous();
     const int y0 = blockIdx.x * rows, o = blockIdx.y, plane = blockIdx.z;  // plane: chunk-local pair*2 + img
     const int w2 = g.w2;
     const int nr = min(rows, g.h2 - y0);

@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
 #include <functional>
 #include <map>
 #include <memory>
@@ -228,6 +229,17 @@ inline void check_dev_alignment(const iqm_pair *pairs, int n) {
 // Copies `bytes` from host memory to `dst` (grown as needed) on the context stream, staging
 // through the pinned ring; returns the device pointer.
 void *upload_bytes(iqm_ctx *ctx, DevBuf &dst, const void *src, size_t bytes);
+
+// upload_bytes into the context's descriptor buffer, followed by n counters that are 0 when the next kernel
+// runs: one copy brings both, and every kernel that counts sets its counter back to 0.
+inline void *upload_with_counters(iqm_ctx *ctx, const void *src, size_t bytes, int n, unsigned *&counters) {
+    const size_t at = (bytes + 15) & ~size_t(15);
+    std::vector<uint8_t> all(at + sizeof(unsigned) * size_t(n));
+    std::memcpy(all.data(), src, bytes);
+    auto *d = static_cast<uint8_t *>(upload_bytes(ctx, ctx->desc, all.data(), all.size()));
+    counters = reinterpret_cast<unsigned *>(d + at);
+    return d;
+}
 
 // Makes at least n side streams (with one join event each) and the fork event exist on the context.
 void side_streams(iqm_ctx *ctx, int n);

@@ -407,14 +407,9 @@ void ssim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, const iqm_ss
                      uintptr_t(q.row_bytes)) & 15u) == 0;
         total += d.ntiles;
     }
-    auto *d_desc = static_cast<SsimPairDev *>(
-        iqm::upload_bytes(ctx, ctx->desc, hd.data(), sizeof(SsimPairDev) * n));
-    const size_t part_bytes = (sizeof(double) * total + 255) & ~size_t(255);
-    const size_t cnt_bytes = (sizeof(unsigned) * n + 255) & ~size_t(255);
-    auto *scr = static_cast<uint8_t *>(ctx->scratch.get(part_bytes + cnt_bytes, ctx->stream));
-    auto *counters = reinterpret_cast<unsigned *>(scr + part_bytes);
-    IQM_CHECK_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned) * n, ctx->stream));
-    iqm::timing_mark(ctx, nullptr);
+    unsigned *counters = nullptr;
+    auto *d_desc = static_cast<SsimPairDev *>(iqm::upload_with_counters(ctx, hd.data(), sizeof(SsimPairDev) * n, n, counters));
+    auto *scr = static_cast<uint8_t *>(ctx->scratch.get(sizeof(double) * total, ctx->stream));
     SsimArgs a{};
     a.pairs = d_desc;
     a.npairs = n;
