@@ -938,7 +938,9 @@ void plane_size(int w, int h, int F, int &w2, int &h2) {  // src/gpu/fsim/fsim.c
 }
 
 constexpr size_t SMEM_CAP = 200 * 1024;
-constexpr int kFsimStreams = 8;  // plane-size groups in flight at once
+// Plane-size groups in flight at once.  24 uneven pairs with 4 / 8 / 12 / 16 / 24: 4576 / 4427 / 4286 / 4231 /
+// 4341 us.
+constexpr int kFsimStreams = 16;
 constexpr bool kOverlapChunks = true;  // rotate inverse-pass chunks over several streams
 // Streams (and buffers) the chunks rotate over: two fill each other's partial waves; three or four
 // measured the same.
