@@ -130,7 +130,8 @@ bool reg_plan(int n, RegFft &best, int &kind) {
     auto consider = [&](bool blue, int p1, int p2, int p3, int k) {
         if ((long long)p1 * p2 * p3 > REG_MAX_POINTS) return;
         const RegFft F = build(n, blue, p1, p2, p3);
-        const long long c = reg_cost(F);
+        // kernels of 80 registers a thread keep half as many warps more resident than those of 128
+        const long long c = reg_cost(F) * (k == REG_DIRECT_32 || k == REG_BLUE_2 ? 5 : 4);
         if (best_cost < 0 || c < best_cost) {
             best_cost = c;
             best = F;
@@ -141,8 +142,10 @@ bool reg_plan(int n, RegFft &best, int &kind) {
         for (int p2 = 1; p2 <= 32; p2++) {
             const int k = p1 <= 24 && p2 <= 24 ? REG_DIRECT_24 : REG_DIRECT_32;
             if (p1 * p2 == n && reg_radix_ok(k, 0, p1) && reg_radix_ok(k, 1, p2)) consider(false, p1, p2, 1, k);
-            if (p1 * p2 >= 2 * n - 1 && reg_radix_ok(REG_BLUE_2, 1, p1) && reg_radix_ok(REG_BLUE_2, 1, p2))
-                consider(true, p1, p2, 1, REG_BLUE_2);
+            if (p1 * p2 >= 2 * n - 1) {
+                const int kb = p1 <= 24 && p2 <= 24 ? REG_BLUE_24 : REG_BLUE_2;
+                if (reg_radix_ok(kb, 1, p1) && reg_radix_ok(kb, 1, p2)) consider(true, p1, p2, 1, kb);
+            }
             if (p1 > 20 || !reg_radix_ok(REG_THREE, 1, p2)) continue;
             for (int p3 = 4; p3 <= 20; p3++) {
                 if (!reg_radix_ok(REG_THREE, 1, p3)) continue;

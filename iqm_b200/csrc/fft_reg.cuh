@@ -229,7 +229,7 @@ __device__ __forceinline__ void reg_last(const RegFft &F, const RegStep &S, cons
 }
 
 // Kinds of plan a kernel is compiled for, so that each holds the code and registers of its own radices.
-enum RegKind { REG_DIRECT_24 = 0, REG_DIRECT_32 = 1, REG_BLUE_2 = 2, REG_THREE = 3, REG_KINDS = 4 };
+enum RegKind { REG_DIRECT_24 = 0, REG_DIRECT_32 = 1, REG_BLUE_2 = 2, REG_THREE = 3, REG_BLUE_24 = 4, REG_KINDS = 5 };
 
 // Radices the steps of each kind implement.  First steps take any radix up to the kind's largest; the
 // others leave out the larger primes, which a plan puts first.
@@ -245,6 +245,8 @@ __host__ __device__ constexpr bool reg_radix_ok(int kind, int where /* 0 first, 
                               : p >= 7 && p <= 32 && p != 17 && p != 19 && p != 23 && p != 29 && p != 31;
         case REG_BLUE_2:
             return smooth || p == 24 || p == 25 || p == 27 || p == 28 || p == 30 || p == 32;
+        case REG_BLUE_24:
+            return smooth || p == 24;
         default:
             return where == 0 ? p >= 2 && p <= 20 : smooth || small;
     }
@@ -276,7 +278,7 @@ __device__ __forceinline__ void reg_fft(const RegFft &F, const Lay &lay, float2 
         with_radix<KIND, 0>(F.st[0].radix, [&](auto P) { reg_first<decltype(P)::value, false>(F, lay, sm, ld); });
         __syncthreads();
         with_radix<KIND, 1>(F.st[1].radix, [&](auto P) { reg_last<decltype(P)::value, false, true>(F, F.st[1], lay, sm, st); });
-    } else if constexpr (KIND == REG_BLUE_2) {
+    } else if constexpr (KIND == REG_BLUE_2 || KIND == REG_BLUE_24) {
         with_radix<KIND, 0>(F.st[0].radix, [&](auto P) { reg_first<decltype(P)::value, true>(F, lay, sm, ld); });
         __syncthreads();
         with_radix<KIND, 1>(F.st[1].radix, [&](auto P) { reg_middle<decltype(P)::value, true, true>(F, F.st[1], lay, sm); });

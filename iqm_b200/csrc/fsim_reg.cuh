@@ -53,6 +53,7 @@ inline void with_kind(int kind, F &&f) {
         case REG_DIRECT_24: f(std::integral_constant<int, REG_DIRECT_24>{}); break;
         case REG_DIRECT_32: f(std::integral_constant<int, REG_DIRECT_32>{}); break;
         case REG_BLUE_2: f(std::integral_constant<int, REG_BLUE_2>{}); break;
+        case REG_BLUE_24: f(std::integral_constant<int, REG_BLUE_24>{}); break;
         default: f(std::integral_constant<int, REG_THREE>{}); break;
     }
 }
@@ -60,6 +61,6 @@ inline void with_kind(int kind, F &&f) {
 // Threads a kernel of a kind may be launched with.
 constexpr int reg_most_threads(int) { return 256; }
 // CTAs of that many threads an SM has to hold: 80 registers a thread serve radices up to 24, 128 the rest.
-constexpr int reg_min_ctas(int kind) { return kind == REG_DIRECT_24 || kind == REG_THREE ? 3 : 2; }
+constexpr int reg_min_ctas(int kind) { return kind == REG_DIRECT_32 || kind == REG_BLUE_2 ? 2 : 3; }
 
 }  // namespace iqm
