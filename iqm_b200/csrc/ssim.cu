@@ -30,6 +30,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "iqm_internal.cuh"
 
@@ -187,12 +188,12 @@ struct Chunk {
     }
 };
 
-// Bound by the FMA pipe (60% busy) and instruction issue (58%): 144 instructions a pixel pair, of which 47
-// are the packed taps of both passes.  Four CTAs per SM at 124 registers, 16 1080p pairs: 236 us, against
-// 397 us for the form before it (a column a thread, eleven loads and squares per pixel, the row loop
+// Bound by the FMA pipe and instruction issue: of the instructions a pixel pair takes, 47 are the packed taps
+// of both passes.  Four CTAs per SM at 126 registers, 16 1080p pairs: 213 us (236 us with a row's tests in
+// every row instead of once a step), against 397 us for the form before it (a column a thread, eleven loads and squares per pixel, the row loop
 // unrolled over the window, a barrier a row; 297 instructions a pixel pair); five CTAs at 96 registers
 // spill, 253 us.  The split-precision tensor-core form took 23.1 us a 1080p pair and the single-product
-// one 15.6 us where this takes 14.7, so every form asked for computes here.
+// one 15.6 us where this takes 13.3, so every form asked for computes here.
 template <int R>
 __global__ void __launch_bounds__(NT, 4) ssim_kernel(SsimArgs args) {
     constexpr int K = 2 * R + 1;
@@ -240,8 +241,10 @@ __global__ void __launch_bounds__(NT, 4) ssim_kernel(SsimArgs args) {
     long long sum = 0;   // and of the strip, in units of 2^-26
     double other = 0.0;  // sums that are no such numbers: k1 or k2 of 0 over flat areas
     auto pool = [&] {
-        if (fabsf(acc) < 16.0f) sum += __float2int_rn(acc * 67108864.0f);
-        else other += acc;
+        if (pool_x) {
+            if (fabsf(acc) < 16.0f) sum += __float2int_rn(acc * 67108864.0f);
+            else other += acc;
+        }
         acc = 0.f;
     };
 
@@ -292,37 +295,51 @@ __global__ void __launch_bounds__(NT, 4) ssim_kernel(SsimArgs args) {
             for (int j = 0; j < 4; j++) sm.h[warp][column_at(4 * lane + j)] = make_float4(hm[j].x, hm[j].y, hs[j].x, hs[j].y);
         }
         __syncthreads();
+        const int yo = yr + RSTEP * s - R;  // the output row that the step's first row completes
+        // vertical taps; rows(plain): every row of the step completes an output row that is pooled, under a
+        // whole window, and no map is wanted
+        auto rows = [&](auto plain) {
 #pragma unroll
-        for (int i = 0; i < RSTEP; i++) {
-            const float4 h = sm.h[i][column_at(tid)];
-            const float2 h1 = make_float2(h.x, h.y), h2 = make_float2(h.z, h.w);
-            const float2 mm = __ffma2_rn(tap(K - 1), h1, am[0]), ms = __ffma2_rn(tap(K - 1), h2, as[0]);
+            for (int i = 0; i < RSTEP; i++) {
+                const float4 h = sm.h[i][column_at(tid)];
+                const float2 h1 = make_float2(h.x, h.y), h2 = make_float2(h.z, h.w);
+                const float2 mm = __ffma2_rn(tap(K - 1), h1, am[0]), ms = __ffma2_rn(tap(K - 1), h2, as[0]);
 #pragma unroll
-            for (int k = 0; k < K - 2; k++) {
-                am[k] = __ffma2_rn(tap(K - 2 - k), h1, am[k + 1]);
-                as[k] = __ffma2_rn(tap(K - 2 - k), h2, as[k + 1]);
+                for (int k = 0; k < K - 2; k++) {
+                    am[k] = __ffma2_rn(tap(K - 2 - k), h1, am[k + 1]);
+                    as[k] = __ffma2_rn(tap(K - 2 - k), h2, as[k + 1]);
+                }
+                am[K - 2] = __fmul2_rn(tap(0), h1);
+                as[K - 2] = __fmul2_rn(tap(0), h2);
+                const int y = yo + i;
+                float wy = gsum;
+                if constexpr (!decltype(plain)::value) {
+                    if (y < y0 || y >= y1) continue;  // uniform, as all branches on y
+                    if (y < R || y >= H - R) {
+                        wy = 0.f;
+#pragma unroll
+                        for (int k = 0; k < K; k++) wy += (y + k - R >= 0 && y + k - R < H) ? tap(k).x : 0.f;
+                    }
+                }
+                const float inv = rwx * iqm::rcp_approx(wy);
+                const float2 sh = __fmul2_rn(mm, make_float2(inv, inv));  // shifted means
+                const float varu = fmaf(ms.x, inv, -sh.x * sh.x), varv = fmaf(ms.y, inv, -sh.y * sh.y);
+                const float2 mu = __fadd2_rn(sh, c), mu2 = __fmul2_rn(mu, mu);
+                const float num = fmaf(0.5f, mu2.x - mu2.y, args.c1) * fmaf(0.5f, varu - varv, args.c2);
+                const float den = fmaf(0.5f, mu2.x + mu2.y, args.c1) * fmaf(0.5f, varu + varv, args.c2);
+                // den >= c1 c2 > 0; a rounded product, so that no path adds it unrounded to the pooled sum
+                const float ssim = __fmul_rn(num, iqm::rcp_approx(den));
+                if constexpr (decltype(plain)::value) {
+                    acc += ssim;
+                } else {
+                    if (P.map && x < W) P.map[(long long)y * W + x] = ssim;
+                    if (y >= R && y <= H - R) acc += ssim;
+                }
+                if (((i - 2 * R) & 3) == 3) pool();  // y & 3 == 3: strips start at multiples of 4
             }
-            am[K - 2] = __fmul2_rn(tap(0), h1);
-            as[K - 2] = __fmul2_rn(tap(0), h2);
-            const int y = yr + RSTEP * s + i - R;  // the output row that this row completes
-            if (y < y0 || y >= y1) continue;       // uniform
-            float wy = gsum;
-            if (y < R || y >= H - R) {
-                wy = 0.f;
-#pragma unroll
-                for (int k = 0; k < K; k++) wy += (y + k - R >= 0 && y + k - R < H) ? tap(k).x : 0.f;
-            }
-            const float inv = rwx * iqm::rcp_approx(wy);
-            const float2 sh = __fmul2_rn(mm, make_float2(inv, inv));  // shifted means
-            const float varu = fmaf(ms.x, inv, -sh.x * sh.x), varv = fmaf(ms.y, inv, -sh.y * sh.y);
-            const float2 mu = __fadd2_rn(sh, c), mu2 = __fmul2_rn(mu, mu);
-            const float num = fmaf(0.5f, mu2.x - mu2.y, args.c1) * fmaf(0.5f, varu - varv, args.c2);
-            const float den = fmaf(0.5f, mu2.x + mu2.y, args.c1) * fmaf(0.5f, varu + varv, args.c2);
-            const float ssim = num * iqm::rcp_approx(den);  // den >= c1 c2 > 0
-            if (P.map && x < W) P.map[(long long)y * W + x] = ssim;
-            if (y >= R && y <= H - R) acc += pool_x ? ssim : 0.f;
-            if (((i - 2 * R) & 3) == 3) pool();  // y & 3 == 3: strips start at multiples of 4
-        }
+        };
+        if (!P.map && yo >= max(y0, R) && yo + RSTEP <= min(y1, H - R)) rows(std::true_type{});
+        else rows(std::false_type{});
         if (s + 1 < steps) {
             first.store(sm, H, shift);
             if (tid < EXTRA) second.store(sm, H, shift);
@@ -348,7 +365,7 @@ void launch_ssim(const SsimArgs &a, int total_tiles, cudaStream_t s) {
 // least estimated time, a tile's rows with its halo (and about a dozen rows' worth of set-up) times the
 // rounds of two CTAs per SM that it takes.  The values of an image do not depend on the choice.  Strips
 // of 8 / 16 / 32 / 64 / 128 rows: one 512x512 pair 15.2 / 15.5 / 19.6 / 27.5 / 43.5 us, 16 1080p pairs
-// 504 / 350 / 273 / 238 / 236 us.
+// 504 / 350 / 273 / 238 / 236 us (before steps without row tests, which took 236 to 213).
 int strip_rows(const iqm_pair *pairs, int n, int R) {
     int best = SHIFT_ROWS;
     double best_cost = 0.0;
