@@ -49,35 +49,18 @@ WORKLOADS = {
     "msvd": ("msvd_1080p_rgb", "rgb_blockquant_pair", 1),
 }
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of each metric's dominant
-# kernel from an ncu capture of this benchmark, with the pairs that launch processed; the summaries
-# under profiles/ give the commands.  Scaled by pairs per launch when the live launch differs.
+# kernel from an ncu capture, with the pairs that launch processed; the summaries are under
+# profiles/.  Scaled by pairs per launch when the live launch differs.
 TRAFFIC = {
-    # ssim_kernel, 32 pairs: 568,007,424 B read + 3,266,560 B written (profiles/ssim_kernel_1080p.md)
-    "ssim": {"kernel": "ssim_kernel", "bytes_per_launch": 571273984, "pairs_per_launch": 32},
-    # fsim_inv_cols_kernel, one chunk of 2 pairs: 10,389,760 + 12,827,904 B (profiles/fsim_inv_cols_kernel_1080p.md)
-    "fsim": {"kernel": "fsim_inv_cols_kernel", "bytes_per_launch": 23217664, "pairs_per_launch": 2},
-    # flip_vcols_kernel, 16 pairs: 1,628,939,776 + 18,826,752 B (profiles/flip_vcols_kernel_1080p.md)
-    "flip": {"kernel": "flip_vcols_kernel", "bytes_per_launch": 1647766528, "pairs_per_launch": 16},
-    # msvd_block_kernel, 32 pairs: 528,075,776 + 6,771,712 B (profiles/msvd_block_kernel_1080p.md)
-    "msvd": {"kernel": "msvd_block_kernel", "bytes_per_launch": 534847488, "pairs_per_launch": 32},
+    # ssim_kernel, 8 pairs: 133.8 MB read + 3.7 MB written (profiles/ssim_kernel_1080p.md)
+    "ssim": {"kernel": "ssim_kernel", "bytes_per_launch": 137500000, "pairs_per_launch": 8},
+    # fsim_inv_rows_reg, 8 pairs: 265.5 MB read + 72.3 MB written (profiles/fsim_inverse_passes.md)
+    "fsim": {"kernel": "fsim_inv_rows_kernel", "bytes_per_launch": 337900000, "pairs_per_launch": 8},
+    # flip_kernel, 4 pairs: 67.8 MB read + 3.3 MB written (profiles/flip_kernel_1080p.md)
+    "flip": {"kernel": "flip_kernel", "bytes_per_launch": 71100000, "pairs_per_launch": 4},
+    # msvd_block_kernel, 8 pairs: 131.8 MB read + 3.8 MB written (profiles/msvd_block_kernel_1080p.md)
+    "msvd": {"kernel": "msvd_block_kernel", "bytes_per_launch": 135600000, "pairs_per_launch": 8},
 }
-# Executed tensor-core work of the mixed FSIM forms on 480x270 planes (1080p and 4K pairs): per pair
-# 32 inverse transforms of each of the 480 columns (270 = 15 x 18: 27 m16n8k16 tiles) and of each
-# of the 270 rows (480 = 16 x 30: 48 tiles), 2 * 16 * 8 * 16 = 4096 flops a tile, times the products
-# per tile (3 with split-precision operands, 1 with single FP16 operands).
-# The mixed SSIM forms run one CTA per 64x64 output tile: 4 warps, each with 5 x 16 horizontal and
-# 4 x 16 vertical m16n8k16 tiles (4 moments x 2 n-tiles x 2 k-steps per 16-row block).
-MMA_PRODUCTS = {"mixed": 3, "mixed_fast": 1}
-
-
-def mma_tiles_per_pair(kernel, w, h):
-    if kernel == "fsim_inv_cols_mma_kernel":
-        return 32 * 480 * 27
-    if kernel == "fsim_inv_rows_mma_kernel":
-        return 32 * 270 * 48
-    if kernel == "ssim_mma_kernel":
-        return -(-w // 64) * -(-h // 64) * 4 * (80 + 64)
-    return 0
 
 
 def workload_name(metric):
@@ -102,8 +85,7 @@ def parse():
                          "CUDA-graph batch plan")
     ap.add_argument("--distinct", type=int, default=4, help="distinct synthetic pairs (replicated to --pairs)")
     ap.add_argument("--precision", default="fp32", choices=["fp32", "mixed", "mixed_fast"],
-                    help="FSIM and SSIM form: FP32, or the tensor-core forms with FP16 operands "
-                         "(split-precision hi + lo products, or single products)")
+                    help="FSIM and SSIM form asked for (all compute FP32)")
     ap.add_argument("--flip-monitor", default="3840,0.7,0.7",
                     help="FLIP viewing set-up RES,DISTANCE,WIDTH (default 67.02 pixels per degree)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
@@ -486,8 +468,6 @@ def main():
         pass
     hbm_peak = float(peaks.get("hbm_gbs", 6650.0))
     peak_note = "measured" if "hbm_gbs" in peaks else "fallback"
-    tensor_peak = float(peaks.get("bf16_tflops", 1590.0))
-    tensor_note = "measured" if "bf16_tflops" in peaks else "fallback"
 
     B = args.pairs or (32 if SIZE == "1080p" else 64)
     host_pairs = make_pairs(metric, min(args.distinct if SIZE == "1080p" else min(args.distinct, 2), B))
@@ -546,9 +526,9 @@ def main():
     ms_per_step = ms / args.steps
     value = world * B / (ms_per_step / 1e3)
 
-    # FSIM and SSIM: the three forms (plain FP32, tensor-core split-precision, tensor-core single
-    # products) on the same device buffers, timed the same way, with their scores of the distinct
-    # pairs kept for the error against the FP64 oracle (reported with the CPU baseline)
+    # FSIM and SSIM: the three forms a caller can ask for, on the same device buffers and timed the
+    # same way, with their scores of the distinct pairs kept for the error against the FP64 oracle
+    # (reported with the CPU baseline)
     forms, form_scores = None, {}
     if metric in ("fsim", "ssim"):
         forms = {}
@@ -604,19 +584,6 @@ def main():
             "avg_launch_us": avg_s * 1e6, "kernel_share": ktimes[kname][1] / ktotal,
             "pipeline_frac": alg_bytes / (ms_per_step / 1e3) / 1e9 / hbm_peak,
             "timing": "CUDA events on the library stream around every launch, second pass of the K steps"}
-    if metric in ("fsim", "ssim") and args.precision in MMA_PRODUCTS:
-        # tensor pipe of the tensor-core kernels: executed MMA flops per launch / average launch time
-        tens = {}
-        for k in ("fsim_inv_cols_mma_kernel", "fsim_inv_rows_mma_kernel", "ssim_mma_kernel"):
-            tiles = mma_tiles_per_pair(k, W, H)
-            if k not in ktimes:
-                continue
-            n_l, t_ms = ktimes[k]
-            flops = B * args.steps * tiles * 4096 * MMA_PRODUCTS[args.precision] / max(1, n_l)
-            achieved_t = flops / (t_ms / max(1, n_l) / 1e3) / 1e12
-            tens[k] = {"achieved": achieved_t, "peak": tensor_peak, "unit": "TFLOP/s", "frac": achieved_t / tensor_peak,
-                       "flops_per_launch": flops, "peak_source": tensor_note + " dense bf16 (burst)"}
-        roof["tensor"] = tens
     if metric == "flip":
         # FLIP is bound by FP32 arithmetic: the SIMT fraction of its filter taps.  Per pixel pair:
         # the CSF prefilter, 3 channels x 2 images x (horizontal + vertical) taps of 2 rc + 1, and
