@@ -22,3 +22,13 @@ def test_fsim_plan_kinds_match_oracle(rt, o64, h, w):
     assert abs(r.fsim - want[0]) <= TOL and abs(r.fsimc - want[1]) <= TOL, (r, want)
     batch = f.compute_batch([(a, b), (b, a), (a, b)])
     assert tuple(batch[0]) == (r.fsim, r.fsimc) == tuple(batch[2])
+
+
+# rows whose four scales come within the row kernel's static shared memory (1 KB) of the 48 KB that a launch
+# may use unasked
+@pytest.mark.parametrize("h,w", [(40, 643), (40, 680), (40, 728), (40, 736), (40, 765), (40, 1360), (40, 1404), (40, 1500)])
+def test_fsim_rows_at_the_default_shared_memory(rt, o64, h, w):
+    a, b = synth.rgb_gain_pair(h, w, config=1, pair=(h + w) % 11)
+    r = iqm_b200.FSIM(rt).compute_metric(a, b)
+    want = o64.fsim(a, b)
+    assert abs(r.fsim - want[0]) <= TOL and abs(r.fsimc - want[1]) <= TOL, (r, want)
