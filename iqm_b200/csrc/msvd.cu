@@ -175,9 +175,23 @@ __device__ __forceinline__ void bidiagonal_step(float2 (&c)[8][4], float (&d)[8]
 // State of the quotient-difference iteration on the squares q of the diagonal and e of the superdiagonal.
 struct QdState {
     float q[8], e[7];
-    float sigma;   // shifts applied so far: an eigenvalue is sigma + its q
-    float s1, s2;  // sums of 1 / x and 1 / x^2 over the eigenvalues of all rows but the last swept one
+    float sigma;     // shifts applied so far: an eigenvalue is sigma + its q
+    float s1, s2;    // sums of 1 / x and 1 / x^2 over the eigenvalues of all rows but the last swept one
+    bool converged;  // no value ran out of sweeps
 };
+
+// No e goes below this.  An exact 0 would split the matrix, and a pivot of 0 above it (a block whose first
+// row and column are black) would make the step across it 0 / 0 and lose the value behind it; with it a
+// pivot of 0 passes its neighbour's q on through e and moves down a row, and sweeps of split matrices bring
+// the smallest value to the end like any other.  As a superdiagonal element it is 1e-10, which moves no
+// singular value by more than that.
+constexpr float kSmallestE = 1e-20f;
+// The last row splits off below this: as a superdiagonal element 1e-4, which is also the most that leaving it
+// out can move a singular value (and moves it by its square over twice the gap to the next one).  A bound
+// that grows with the value, e <= 1e-5 x, let close values move by up to 1e-2; asking for the gap as well
+// cost more than the sweep that the last digits take (209 us for 16 1080p pairs; with gaps 223 and above).
+constexpr float kNegligibleE = 1e-8f;
+constexpr int kMostSweeps = 24;  // of one value; about three in 10^5 noisy diagonal blocks need more
 
 // Laguerre's lower bound of the smallest of m positive numbers whose reciprocals and their squares sum to
 // s1 and s2, a little less; 0 where the sums are not usable.
@@ -188,26 +202,27 @@ __device__ __forceinline__ float laguerre_shift(float m, float s1, float s2) {
 }
 
 // Finds the smallest eigenvalue of the leading M rows and leaves it in q[M - 1] + sigma: shifted
-// differential qd sweeps until the last superdiagonal element no longer moves a singular value by 1e-5.
+// differential qd sweeps until the last row splits off.
 // Every sweep also carries the first two derivatives of its pivots by the shift, which give the sums over
 // 1 / x and 1 / x^2 of the swept matrix's eigenvalues and with them the next shift; the sums without the
 // last pivot are those of the matrix that is left when the last row splits off.
 template <int M>
 __device__ __forceinline__ void qd_smallest(QdState &z) {
-    constexpr float kTiny = 1e-10f;
     float tau = M == 8 ? 0.0f : laguerre_shift(float(M), z.s1, z.s2);
 #pragma unroll 1
-    for (int it = 0; it < 24; it++) {
-        const float el = z.e[M - 2];
-        if (el * el <= fmaxf(1e-10f * (z.sigma + z.q[M - 1]), 1e-18f)) break;
+    for (int it = 0; z.e[M - 2] > kNegligibleE; it++) {
+        if (it == kMostSweeps) {
+            z.converged = false;
+            break;
+        }
         float Q[M], E[M - 1];
         float dd = z.q[0] - tau, low = dd, d1 = -1.0f, d2 = 0.0f, s1 = 0.0f, s2 = 0.0f;
 #pragma unroll
         for (int i = 0; i < M - 1; i++) {
-            Q[i] = dd + z.e[i];
-            const float r = iqm::rcp_approx(fmaxf(Q[i], kTiny));
+            Q[i] = dd + z.e[i];  // at least kSmallestE unless the shift is rejected below
+            const float r = iqm::rcp_approx(Q[i]);
             const float t = z.q[i + 1] * r;
-            E[i] = z.e[i] * t;
+            E[i] = fmaxf(z.e[i] * t, kSmallestE);
             const float a = d1 * r, w = E[i] * r;
             s1 -= a;
             s2 = fmaf(-d2, r, fmaf(a, a, s2));
@@ -225,7 +240,7 @@ __device__ __forceinline__ void qd_smallest(QdState &z) {
             z.sigma += tau;
             z.s1 = s1;
             z.s2 = s2;
-            const float r = iqm::rcp_approx(fmaxf(dd, kTiny)), a = d1 * r;
+            const float r = iqm::rcp_approx(fmaxf(dd, kSmallestE)), a = d1 * r;
             tau = laguerre_shift(float(M), s1 - a, fmaf(-d2, r, fmaf(a, a, s2)));
         } else {
             tau = 0.0f;  // the shift passed the smallest eigenvalue: sweep again without one
@@ -234,14 +249,12 @@ __device__ __forceinline__ void qd_smallest(QdState &z) {
     z.q[M - 1] += z.sigma;
 }
 
-// Singular values (descending) of the 8x8 matrix whose columns are c[0..7]; c is destroyed.
+// Singular values of the 8x8 matrix whose columns are c[0..7], in no order; c is destroyed.  False where
+// the iteration ran out of sweeps.
 // Householder reflections to bidiagonal form, then the singular values of that by shifted differential
 // qd sweeps (K. V. Fernando and B. N. Parlett, "Accurate singular values and differential qd algorithms",
-// 1994), smallest first, with Laguerre's shifts.  On 8.1k blocks of an 8x8-quantised image the largest
-// deviation from double-precision singular values is 4.5e-4 and the RMS 3.9e-5 (values up to 2040); the
-// one-sided Jacobi method that this replaced had 6.3e-4 and 6.6e-5 and took about twice the time, six to
-// eight sweeps of 28 rotations.
-__device__ __forceinline__ void svd8_values(float2 (&c)[8][4], float s[8]) {
+// 1994), smallest first, with Laguerre's shifts.
+__device__ __forceinline__ bool svd8_qd(float2 (&c)[8][4], float (&s)[8]) {
     QdState z;
     {
         float d[8], e[7];
@@ -256,9 +269,10 @@ __device__ __forceinline__ void svd8_values(float2 (&c)[8][4], float s[8]) {
 #pragma unroll
         for (int i = 0; i < 8; i++) z.q[i] = d[i] * d[i];
 #pragma unroll
-        for (int i = 0; i < 7; i++) z.e[i] = e[i] * e[i];
+        for (int i = 0; i < 7; i++) z.e[i] = fmaxf(e[i] * e[i], kSmallestE);
     }
     z.sigma = z.s1 = z.s2 = 0.0f;
+    z.converged = true;
     qd_smallest<8>(z);
     qd_smallest<7>(z);
     qd_smallest<6>(z);
@@ -269,6 +283,91 @@ __device__ __forceinline__ void svd8_values(float2 (&c)[8][4], float s[8]) {
     z.q[0] += z.sigma;
 #pragma unroll
     for (int i = 0; i < 8; i++) s[i] = z.q[i] > 1e-30f ? sqrt_newton(z.q[i]) : 0.0f;
+    return z.converged;
+}
+
+// <ci, cj> over the 8 rows
+__device__ __forceinline__ float dot8(const float2 (&ci)[4], const float2 (&cj)[4]) {
+    float2 q = iqm::mul2(ci[0], cj[0]);
+#pragma unroll
+    for (int k = 1; k < 4; k++) q = iqm::fma2(ci[k], cj[k], q);
+    return q.x + q.y;
+}
+
+// The same by one-sided Jacobi rotations, which need no shifts and converge on every block: for those that
+// ran out of sweeps.  Each pair of columns is rotated so that they become orthogonal, until no inner product
+// is above FP32's rounding of the two norms; the final norms are summed in FP64.
+__device__ __forceinline__ void svd8_jacobi(float2 (&c)[8][4], float (&s)[8]) {
+    const float eps2 = 16.0f * FLT_EPSILON * FLT_EPSILON;
+#pragma unroll 1
+    for (int sweep = 0; sweep < 60; sweep++) {
+        bool changed = false;
+#pragma unroll
+        for (int i = 0; i < 7; i++) {
+#pragma unroll
+            for (int j = i + 1; j < 8; j++) {
+                const float p = dot8(c[i], c[j]), ni = dot8(c[i], c[i]), nj = dot8(c[j], c[j]);
+                // inner products below 1e-15 count as 0, so that columns of rounding noise end too
+                if (p * p > fmaxf(eps2 * ni * nj, 1e-30f)) {
+                    const float zeta = (nj - ni) / (2.0f * p), az = fabsf(zeta);
+                    // tan(theta): smaller root of t^2 + 2 zeta t - 1 = 0 (1 / (2 zeta) once zeta^2 overflows)
+                    const float t = copysignf(1.0f, zeta) / (az < 1e18f ? az + sqrtf(fmaf(zeta, zeta, 1.0f)) : 2.0f * az);
+                    const float cs = 1.0f / sqrtf(fmaf(t, t, 1.0f)), sn = cs * t;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const float2 xi = c[i][k], xj = c[j][k];
+                        c[i][k] = iqm::fma2(iqm::dup2(cs), xi, iqm::mul2(iqm::dup2(-sn), xj));
+                        c[j][k] = iqm::fma2(iqm::dup2(sn), xi, iqm::mul2(iqm::dup2(cs), xj));
+                    }
+                    changed = true;
+                }
+            }
+        }
+        if (!changed) break;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        double q = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            q = fma(double(c[i][k].x), double(c[i][k].x), q);
+            q = fma(double(c[i][k].y), double(c[i][k].y), q);
+        }
+        s[i] = float(sqrt(q));
+    }
+}
+
+// Out of line and from the pixels again, so that this rare path holds no registers of the usual one.
+__device__ __noinline__ void block_values_jacobi(const MsvdPairDev *pairs, int npairs, int slot, int img, float *out) {
+    const MsvdPairDev P = pairs[find_pair(pairs, npairs, slot)];
+    const int local = slot - P.slot_base;
+    float2 c[8][4];
+    float s[8];
+    load_block(img ? P.b : P.a, P.pitch, 8 * (local % P.bw), 8 * (local / P.bw), P.vec_ok, c);
+    svd8_jacobi(c, s);
+#pragma unroll
+    for (int i = 0; i < 8; i++) out[i] = s[i];
+}
+
+// Singular values (descending) of the 8x8 grey block of a slot and image; P is the slot's pair.
+// Over 31 kinds of blocks (noise, text, edges, patches and sparse pixels on black and on white, flat and
+// nearly flat, diagonal and block diagonal ones, of rank one and two; a million each) no value is 7.2e-4 away
+// from its double-precision one, RMS 5e-5 and less (values up to 2040); one-sided Jacobi alone reaches 1.5e-3,
+// RMS 1.3e-4, in more than twice the time, six to eight sweeps of 28 rotations.
+__device__ __forceinline__ void block_values(const MsvdArgs &args, const MsvdPairDev &P, int bx, int by, int slot, int img,
+                                             float (&s)[8]) {
+    bool converged;
+    {
+        float2 c[8][4];
+        load_block(img ? P.b : P.a, P.pitch, 8 * bx, 8 * by, P.vec_ok, c);
+        converged = svd8_qd(c, s);
+    }
+    if (!converged) {
+        float t[8];
+        block_values_jacobi(args.pairs, args.npairs, slot, img, t);
+#pragma unroll
+        for (int i = 0; i < 8; i++) s[i] = t[i];
+    }
     // descending order (sorting network on 8 registers)
 #define IQM_CSWAP(a, b)                         \
     do {                                        \
@@ -292,7 +391,8 @@ __device__ __forceinline__ void svd8_values(float2 (&c)[8][4], float s[8]) {
 // copy of the SVD code serves both images and twice as many blocks are in flight.
 // Bound by instruction issue (72% of the issue slots, FMA pipe 52%, 4.7k instructions a block of one
 // image, about a sixth of them lost to lanes that wait for their warp's slowest qd sweep).  16 1080p
-// pairs: 475 us with Jacobi sweeps, 178 us now; five CTAs per SM at 93 registers 185 us, six at 80 178 us.
+// pairs: 475 us with Jacobi sweeps, 183 us now; five CTAs per SM at 93 registers took 185 us where six at 80
+// took 178 us.
 __global__ void __launch_bounds__(BLOCK_THREADS, 6) msvd_block_kernel(MsvdArgs args) {
     const int slot = (blockIdx.x * BLOCK_THREADS + threadIdx.x) >> 1;
     const int img = threadIdx.x & 1;
@@ -311,10 +411,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 6) msvd_block_kernel(MsvdArgs a
     const unsigned mask = __ballot_sync(0xffffffffu, computed);
     if (computed) {
         {  // one 8x8 block of one image
-            float2 c[8][4];
-            load_block(img ? P.b : P.a, P.pitch, 8 * bx, 8 * by, P.vec_ok, c);
             float s[8];
-            svd8_values(c, s);
+            block_values(args, P, bx, by, slot, img, s);
             float acc = 0.0f;  // shaders/svd/svd.glsl:41-52: float, k = 0..7 in order
 #pragma unroll
             for (int k = 0; k < 8; k++) {
