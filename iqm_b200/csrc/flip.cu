@@ -29,6 +29,7 @@
 
 #include "iqm_internal.cuh"
 #include "packed_f32x2.cuh"
+#include "pooled_sum.cuh"
 
 #define GLSL_PI 3.141592653589
 
@@ -62,7 +63,6 @@ struct FlipPairDev {
     long long pitch;
     int w, h;
     int tiles_x, ntiles, tile_base;
-    int vec_ok;
     long long plane_off;  // offset (floats) of this pair's 12 planes
     long long seg_base;   // first hpass work unit (HROWS rows of one 512-pixel segment) of this pair
 };
@@ -71,10 +71,10 @@ struct FlipArgs {
     const FlipPairDev *pairs;
     int npairs;
     float *planes;
-    double *partials;
+    double *partials;       // one per tile: flip_vpass_kernel
+    iqm::PooledSum *sums;   // one per tile: flip_kernel
     unsigned *counters;
     double *scores;
-    long long total_segs;
     int strip;  // rows of a tile (flip_kernel)
 };
 
@@ -413,6 +413,7 @@ constexpr int FUSED_MAXR = 14;
 constexpr int FW = 64;                 // columns of a strip
 constexpr int FROWS = 14;              // rows of a step: two rounds of pixels, three of row filters
 constexpr int FT_THREADS = 7 * FW;     // a thread a vertical filter and column
+constexpr int MAX_STEPS = 12;          // of a strip
 constexpr int HFILT = 6, VFILT = 7;
 
 // The taps by window position u (row or column y - R + u of output y), zero beyond a filter's own radius,
@@ -524,8 +525,6 @@ __global__ void __launch_bounds__(FT_THREADS, R <= 11 ? 2 : 1) flip_kernel(FlipA
     constexpr int PER_T = (FROWS + GROUPS - 1) / GROUPS;
     extern __shared__ __align__(16) unsigned char flip_smem[];
     Sm &sm = *reinterpret_cast<Sm *>(flip_smem);
-    __shared__ double red[FT_THREADS / 32];
-    __shared__ int is_last;
     const int gt = blockIdx.x;
     const int pi = find_tile(args.pairs, args.npairs, gt);
     const FlipPairDev P = args.pairs[pi];
@@ -554,8 +553,7 @@ __global__ void __launch_bounds__(FT_THREADS, R <= 11 ? 2 : 1) flip_kernel(FlipA
     float2 acc[2 * R];
 #pragma unroll
     for (int k = 0; k < 2 * R; k++) acc[k] = make_float2(0.f, 0.f);
-    long long sum = 0;   // of the pixels' values, in units of 2^-28
-    double other = 0.0;  // values that are no such numbers
+    iqm::PooledSum sum;  // of the pixels' values
     const int steps = (y1 - y0 + 2 * R + FROWS - 1) / FROWS;
     load(0);
     __syncthreads();  // the sRGB table
@@ -612,13 +610,13 @@ __global__ void __launch_bounds__(FT_THREADS, R <= 11 ? 2 : 1) flip_kernel(FlipA
             for (int q = 0; q < VFILT; q++) f[q] = sm.v[(row * VFILT + q) * FW + c];
             const float val = fused_pixel(T, f);
             if (P.map) P.map[size_t(y) * size_t(P.w) + x] = val;
-            if (fabsf(val) < 4.0f) sum += __float2int_rn(val * 268435456.0f);
-            else other += val;
+            sum.add(val);
         }
         __syncthreads();  // the filtered values are read before the next rows are staged
     }
-    // Sums of these are exact in FP64 (up to 2^25 pixels), so the cut into strips does not matter.
-    pool_tile<FT_THREADS>(args, P, pi, gt, double(sum) * (1.0 / 268435456.0) + other, red, is_last);
+    static_assert(FW * FROWS * MAX_STEPS <= 1 << 14, "a tile's values fit a PooledSum");
+    iqm::pool_tiles<FT_THREADS>(sum, args.sums, args.counters, args.scores, pi, gt, P.tile_base, P.ntiles,
+                                double(P.w) * double(P.h));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -769,7 +767,7 @@ FusedTaps fused_taps(const FlipTaps &T, int R) {
 int strip_rows(const std::vector<iqm_pair> &pairs, int R) {
     int best = 0;
     double best_cost = 0.0;
-    for (int steps = 12; FROWS * steps > 2 * R; steps--) {
+    for (int steps = MAX_STEPS; FROWS * steps > 2 * R; steps--) {
         const int s = FROWS * steps - 2 * R;
         double tiles = 0.0;
         for (const iqm_pair &p : pairs) tiles += double(iqm::ceil_div(p.w, FW)) * iqm::ceil_div(p.h, s);
@@ -829,7 +827,6 @@ void flip_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, const iqm_fl
         d.tiles_x = int(iqm::ceil_div(q.w, fused ? FW : VT_COLS));
         d.ntiles = d.tiles_x * int(iqm::ceil_div(q.h, strip));
         d.tile_base = tiles;
-        d.vec_ok = 0;
         d.plane_off = plane_floats;
         d.seg_base = segs;
         tiles += d.ntiles;
@@ -840,15 +837,15 @@ void flip_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, const iqm_fl
     unsigned *counters = nullptr;
     auto *d_desc = static_cast<FlipPairDev *>(iqm::upload_with_counters(ctx, hd.data(), sizeof(FlipPairDev) * n, n, counters));
     const size_t pb = (sizeof(float) * size_t(plane_floats) + 255) & ~size_t(255);
-    auto *base = static_cast<uint8_t *>(ctx->scratch.get(pb + sizeof(double) * tiles, ctx->stream));
+    auto *base = static_cast<uint8_t *>(ctx->scratch.get(pb + sizeof(iqm::PooledSum) * tiles, ctx->stream));
     FlipArgs a{};
     a.pairs = d_desc;
     a.npairs = n;
     a.planes = reinterpret_cast<float *>(base);
     a.partials = reinterpret_cast<double *>(base + pb);
+    a.sums = reinterpret_cast<iqm::PooledSum *>(base + pb);
     a.counters = counters;
     a.scores = d_scores;
-    a.total_segs = segs;
     if (fused) {
         a.strip = strip;
         launch_fused(a, T, std::max(R, FUSED_MINR), tiles, ctx->stream);
