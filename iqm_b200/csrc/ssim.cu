@@ -15,8 +15,8 @@
 //     cov_ab = (var_u - var_v)/4, var_a + var_b = (var_u + var_v)/2;
 //   * the second moments are taken about a per-tile constant (the u, v of the tile's centre
 //     pixel), var = E[(x-c)^2] - E[x-c]^2, which keeps FP32 cancellation ~1e-7 on MSSIM;
-//   * lumas stay whole numbers, 299 R + 581 G + 114 B, so (u, v) and their distance to the constant are
-//     exact in FP32 until the first tap multiplies them;
+//   * lumas stay whole numbers, 299 R + 581 G + 114 B, in units of 2^-18, so (u, v) and their distance to the
+//     constant are exact in FP32 until the first tap multiplies them;
 //   * each CTA owns a 128-column strip and streams down it four rows a step: the rows' (u, v) go to
 //     shared memory, a warp a row filters them horizontally, four neighbouring columns a lane (a
 //     staged value is loaded and squared once for the eleven outputs it serves), and a thread a column
@@ -42,7 +42,7 @@ constexpr int RSTEP = 4;            // rows per step: a warp each in the horizon
 constexpr int UNITS = (TW + 16) / 2;  // staged columns x0-8 .. x0+TW+7 of a row, two to a 16-byte unit
 constexpr int CHUNKS = (TW + 16) / 4; // 4-pixel loads of a row
 constexpr int SHIFT_ROWS = 128;     // rows that share a shift constant; strips divide it
-constexpr float LUMA_UNIT = 255000.0f;  // a luma of 1 in the whole numbers used here
+constexpr float LUMA_UNIT = 255000.0f / 262144.0f;  // a luma of 1 in the units used here: near 1, for the range of c1 and c2
 
 struct Smem {
     float4 uv[RSTEP][UNITS];  // shifted (u, v) of two columns, at unit_at(flat index)
@@ -81,12 +81,12 @@ struct SsimArgs {
 __device__ __forceinline__ int luma_i(uint32_t px, int add) {
     return int(__dp2a_hi(114u, px, __dp2a_lo(299u | 581u << 16, px, unsigned(add))));
 }
-// (u, v) of a pixel pair as 1.5 * 2^23 + value in floats, whose spacing there is 1
+// (u, v) of a pixel pair as 48 + value * 2^-18 in floats, whose spacing there is 2^-18
 __device__ __forceinline__ float2 uv_biased(uint32_t pa, uint32_t pb) {
-    const int a = luma_i(pa, 0x4B400000), b = luma_i(pb, 0);
+    const int a = luma_i(pa, 0x42400000), b = luma_i(pb, 0);
     return make_float2(__int_as_float(a + b), __int_as_float(a - b));
 }
-constexpr float UV_BIAS = 12582912.0f;
+constexpr float UV_BIAS = 48.0f;
 
 __device__ __forceinline__ int find_pair(const SsimPairDev *pairs, int n, int tile) {
     int lo = 0, hi = n - 1;
@@ -327,7 +327,9 @@ __global__ void __launch_bounds__(NT, 4) ssim_kernel(SsimArgs args) {
                 const float2 mu = __fadd2_rn(sh, c), mu2 = __fmul2_rn(mu, mu);
                 const float num = fmaf(0.5f, mu2.x - mu2.y, args.c1) * fmaf(0.5f, varu - varv, args.c2);
                 const float den = fmaf(0.5f, mu2.x + mu2.y, args.c1) * fmaf(0.5f, varu + varv, args.c2);
-                // den >= c1 c2 > 0; a rounded product, so that no path adds it unrounded to the pooled sum
+                // den is about c1 c2 or more, but 0 is possible: k1 or k2 may be 0, and the variances round; inside
+                // the reciprocal's range, 2^-126 to 2^126, as long as c1 c2 is.  A rounded product, so that no path
+                // adds it unrounded to the pooled sum
                 const float ssim = __fmul_rn(num, iqm::rcp_approx(den));
                 if constexpr (decltype(plain)::value) {
                     acc += ssim;
