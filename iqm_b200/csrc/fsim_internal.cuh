@@ -61,7 +61,9 @@ struct FsimGroup {
 };
 
 // A kernel of FSIM's chain may be launched while the one before it in its stream still drains (launch_after);
-// it calls this before it touches memory and goes on when that one's writes are visible.
+// it calls this before it touches memory and goes on when that one's writes are visible.  What another kernel
+// of the chain writes is not read with __ldg, whose memory must not change while the kernel runs: this one runs
+// from its launch on, when that memory is still being written.  Plan tables may be.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Launches a kernel that calls wait_for_previous(): its CTAs are set up during the tail of the stream's

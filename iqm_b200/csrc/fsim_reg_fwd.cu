@@ -22,7 +22,7 @@ fsim_fwd_rows_reg(FsimGroup g, const __grid_constant__ RegFft F, int rows) {
         [&](int seq, int i, int items) {
             const float *a = Y1 + (seq * w2 + i), *b = Y2 + (seq * w2 + i);
             const unsigned d = 4u * unsigned(items);
-            return [=](int r) { return make_float2(__ldg(run_at(b, d, r)), __ldg(run_at(a, d, r))); };
+            return [=](int r) { return make_float2(__ldcg(run_at(b, d, r)), __ldcg(run_at(a, d, r))); };
         },
         [&](int seq, int i, int items) {
             float2 *z0 = Z + (seq * w2 + i);
@@ -52,7 +52,7 @@ fsim_fwd_cols_reg(FsimGroup g, const __grid_constant__ RegFft F, int lc) {
             const float2 *z0 = Z + (i * w2 + column(seq));
             const unsigned d = 8u * unsigned(items * w2);
             return [=](int r) {
-                const float2 z = __ldg(run_at(z0, d, r));
+                const float2 z = __ldcg(run_at(z0, d, r));
                 return make_float2(z.y, z.x);
             };
         },
