@@ -1185,9 +1185,11 @@ Layout layout_for(int G, int chunk, int n, int tiles, int nbuf, int tiled) {
 // empty for most of their time, which costs more than sending the planes through HBM.  32 1080p pairs in
 // budgets of 80 / 160 / 320 / 640 / 1200 MB: 1095 / 1094 / 1050 / 1017 / 1009 us; 32 pairs of 512x512:
 // 520 / 526 / 497 / 495 / 495 us.
+constexpr int kMostChunkPairs = 65535 / 2;  // a chunk's images are the z dimension of its grids
+
 int chunk_pairs(const iqm::FsimTune &t, int G, int n) {
     const size_t budget = size_t(t.chunk_mb > 0 ? t.chunk_mb : 640) << 20;
-    return std::max(1, std::min(G, int(budget / (sizeof(float2) * 32 * size_t(n)))));
+    return std::max(1, std::min({G, kMostChunkPairs, int(budget / (sizeof(float2) * 32 * size_t(n)))}));
 }
 
 void launch_ingest(const FsimGroup &g, int F_uniform, int tiles, cudaStream_t st) {
