@@ -939,7 +939,7 @@ void plane_size(int w, int h, int F, int &w2, int &h2) {  // src/gpu/fsim/fsim.c
 }
 
 constexpr size_t SMEM_CAP = 200 * 1024;
-// Plane-size groups in flight at once.  24 uneven pairs with 4 / 8 / 12 / 16 / 24: 4576 / 4427 / 4286 / 4231 /
+// Plane-size groups in flight at once, at most.  24 uneven pairs with 4 / 8 / 12 / 16 / 24: 4576 / 4427 / 4286 / 4231 /
 // 4341 us.
 constexpr int kFsimStreams = 16;
 constexpr bool kOverlapChunks = true;  // rotate inverse-pass chunks over several streams
@@ -1180,15 +1180,16 @@ Layout layout_for(int G, int chunk, int n, int tiles, int nbuf, int tiled) {
     return L;
 }
 
-// Inverse-pass chunk: the 32 intermediate planes of `chunk` pairs stay within a budget (640 MB unless
-// tuned).  The L2 would hold two 1080p pairs' planes, but launches of a pair or two leave the SMs half
-// empty for most of their time, which costs more than sending the planes through HBM.  32 1080p pairs in
+// Inverse-pass intermediates: the chunks in flight share a budget (640 MB unless tuned), split evenly over the
+// plane-size groups that run at once; a chunk takes as many pairs as their 32 planes each fit its group's
+// part, at least one.  The L2 would hold two 1080p pairs' planes, but launches of a pair or two leave the SMs
+// half empty for most of their time, which costs more than sending the planes through HBM.  32 1080p pairs in
 // budgets of 80 / 160 / 320 / 640 / 1200 MB: 1095 / 1094 / 1050 / 1017 / 1009 us; 32 pairs of 512x512:
 // 520 / 526 / 497 / 495 / 495 us.
+constexpr int kChunkMb = 640;
 constexpr int kMostChunkPairs = 65535 / 2;  // a chunk's images are the z dimension of its grids
 
-int chunk_pairs(const iqm::FsimTune &t, int G, int n) {
-    const size_t budget = size_t(t.chunk_mb > 0 ? t.chunk_mb : 640) << 20;
+int chunk_pairs(size_t budget, int G, int n) {
     return std::max(1, std::min({G, kMostChunkPairs, int(budget / (sizeof(float2) * 32 * size_t(n)))}));
 }
 
@@ -1248,13 +1249,6 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
             const int n = r.P->n;
             if (r.P->reg) r.rs = iqm::reg_shapes(*r.P, ctx->fsim_tune);
             else r.s = shapes_for(*r.P, ctx->fsim_tune);
-            r.chunk = chunk_pairs(ctx->fsim_tune, r.G, n);
-            // More than one chunk: split the budget over two buffers and let consecutive chunks run
-            // on two streams, so one chunk's column pass fills the other's last partial wave.
-            r.overlap = kOverlapChunks && !ctx->timing && r.G > r.chunk;
-            if (r.overlap) r.chunk = std::max(1, r.chunk / kChunkStreams);
-            r.L = layout_for(r.G, r.chunk, n, int(iqm::ceil_div(n, FT)), r.overlap ? kChunkStreams : 1,
-                             r.P->tiled);
             r.F_uniform = hd[kv.second[0]].F;
             for (int i : kv.second)
                 if (hd[i].F != r.F_uniform) r.F_uniform = 0;
@@ -1267,25 +1261,51 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
     // Groups are independent: up to kFsimStreams of them run at once on side streams forked from the
     // context stream and joined back (kept on one stream while per-kernel timing is on).  Each
     // stream reuses one scratch slot for its groups, which it runs in order.
-    const int S = (runs.size() > 1 && !ctx->timing) ? std::min<int>(int(runs.size()), kFsimStreams) : 1;
-    {
-        std::vector<int> order(runs.size());
-        for (size_t i = 0; i < order.size(); i++) order[i] = int(i);
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return runs[a].cost > runs[b].cost; });
+    std::vector<int> order(runs.size());
+    for (size_t i = 0; i < order.size(); i++) order[i] = int(i);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return runs[a].cost > runs[b].cost; });
+    const bool serial = runs.size() == 1 || ctx->timing;
+    iqm::FsimTune t = ctx->fsim_tune;
+    if (!t.chunk_mb) t.chunk_mb = kChunkMb;
+    if (!t.streams) t.streams = kFsimStreams;
+    int S = 1;
+    std::vector<size_t> slot_off;
+    // Slots, chunks and layouts for t; false when nothing could be smaller.
+    auto lay_out = [&] {
+        S = serial ? 1 : std::min<int>(int(runs.size()), t.streams);
+        bool smaller = S > 1 || !t.tight;
         std::vector<double> load(S, 0.0);
-        for (int i : order) {
-            const int sl = int(std::min_element(load.begin(), load.end()) - load.begin());
-            runs[i].slot = sl;
-            load[sl] += runs[i].cost;
-        }
-    }
-    std::vector<size_t> slot_off(S + 1, 0);
-    {
         std::vector<size_t> need(S, 0);
-        for (const auto &r : runs) need[r.slot] = std::max(need[r.slot], r.L.total);
+        for (int i : order) {
+            GroupRun &r = runs[i];
+            r.slot = int(std::min_element(load.begin(), load.end()) - load.begin());
+            load[r.slot] += r.cost;
+            const int n = r.P->n;
+            r.chunk = chunk_pairs((size_t(t.chunk_mb) << 20) / S, r.G, n);
+            smaller |= r.chunk > 1 && t.chunk_mb > 1;
+            // More than one chunk: split the budget over two buffers and let consecutive chunks run
+            // on two streams, so one chunk's column pass fills the other's last partial wave.
+            r.overlap = kOverlapChunks && !ctx->timing && r.G > r.chunk && (r.chunk >= kChunkStreams || !t.tight);
+            if (r.overlap) r.chunk = std::max(1, r.chunk / kChunkStreams);
+            r.L = layout_for(r.G, r.chunk, n, int(iqm::ceil_div(n, FT)), r.overlap ? kChunkStreams : 1, r.P->tiled);
+            need[r.slot] = std::max(need[r.slot], r.L.total);
+        }
+        slot_off.assign(S + 1, 0);
         for (int sl = 0; sl < S; sl++) slot_off[sl + 1] = slot_off[sl] + ((need[sl] + 255) & ~size_t(255));
+        return smaller;
+    };
+    // Where the GPU has too little memory left, half the budget and half the streams, until the scratch fits.
+    uint8_t *base0 = nullptr;
+    for (;;) {
+        const bool smaller = lay_out();
+        base0 = static_cast<uint8_t *>(smaller ? ctx->scratch.try_get(slot_off[S], ctx->stream)
+                                               : ctx->scratch.get(slot_off[S], ctx->stream));
+        if (base0) break;
+        t.chunk_mb = std::max(1, t.chunk_mb / 2);
+        t.streams = (S + 1) / 2;
+        t.tight = true;
     }
-    auto *base0 = static_cast<uint8_t *>(ctx->scratch.get(slot_off[S], ctx->stream));
+    ctx->fsim_used = t;
     std::vector<cudaStream_t> streams(S, ctx->stream);
     bool any_overlap = false;
     for (const auto &r : runs) any_overlap |= r.overlap;

@@ -56,6 +56,19 @@ struct DevBuf {
         cap = want;
         return ptr;
     }
+    // As get, but nullptr when that much memory is not free, without giving the present buffer back.
+    void *try_get(size_t bytes, cudaStream_t s) {
+        if (bytes <= cap) return ptr;
+        size_t avail = 0, total = 0;
+        IQM_CHECK_CUDA(cudaMemGetInfo(&avail, &total));
+        if (bytes + 256 > avail + cap) return nullptr;
+        try {
+            return get(bytes, s);
+        } catch (const Error &e) {
+            if (e.code != IQM_ENOMEM) throw;
+            return nullptr;
+        }
+    }
     void release() {
         if (ptr) cudaFree(ptr);
         ptr = nullptr;
@@ -110,10 +123,12 @@ struct UploadRing {
     }
 };
 
-// Launch-shape choices of the FSIM transform passes (0 / -1 = built-in heuristic).  They change
+// Launch-shape choices of the FSIM transform passes (0 = built-in heuristic).  They change
 // only how work is split over CTAs, never a result bit; batch plans autotune them (plan.cu).
 struct FsimTune {
-    int chunk_mb = 0;     // budget for the inverse-pass intermediates of one chunk of pairs
+    int chunk_mb = 0;     // budget for the inverse-pass intermediates of all chunks in flight
+    int streams = 0;      // plane-size groups in flight, at most
+    bool tight = false;   // memory is short: no second buffer for chunks of one pair
     int rows_per_cta = 0; // rows per CTA of the inverse row pass (1 or 2, if it fits)
 };
 
@@ -131,6 +146,7 @@ struct iqm_ctx {
     int launches = 0;  // kernel launches enqueued by the last entry point
     bool capturing = false;  // a batch plan is capturing the stream into a CUDA graph (plan.cu)
     iqm::FsimTune fsim_tune;
+    iqm::FsimTune fsim_used;  // what the last FSIM enqueue ran with: fsim_tune, or less where memory was short
     // streams that independent work forks onto from `stream` and joins back from (iqm::side_streams)
     std::vector<cudaStream_t> side_streams;
     std::vector<cudaEvent_t> side_events;

@@ -93,15 +93,15 @@ struct iqm_batch_plan {
     std::vector<iqm_pair> pairs;
     double *d_scores = nullptr;
     iqm::DevBuf desc[4], scratch[4];
-    iqm::FsimTune tune;
+    iqm::FsimTune tune;  // FSIM's shapes; after an enqueue, those that it could have the memory for
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int launches = 0;
     std::string info;
 
     // Enqueues every metric of the mask (or only metric index `only`) with the plan's buffers;
-    // returns the kernel launches.
-    int enqueue(const iqm::FsimTune &t, int only = -1) {
+    // returns the kernel launches.  t becomes what FSIM ran with.
+    int enqueue(iqm::FsimTune &t, int only = -1) {
         int total = 0;
         double *out = d_scores;
         const int n = int(pairs.size());
@@ -111,6 +111,7 @@ struct iqm_batch_plan {
                 BorrowBuffers b(ctx, desc[m], scratch[m], t);
                 ctx->launches = 0;
                 enqueue_metric(ctx, m, args, pairs.data(), n, out);
+                if (kMetrics[m] == IQM_METRIC_FSIM) t = ctx->fsim_used;
                 total += ctx->launches;
             }
             out += size_t(kScores[m]) * n;
@@ -119,7 +120,7 @@ struct iqm_batch_plan {
     }
 
     // Milliseconds of one FSIM enqueue with shapes t (after one untimed run that sizes buffers).
-    float time_fsim(const iqm::FsimTune &t, cudaEvent_t e0, cudaEvent_t e1) {
+    float time_fsim(iqm::FsimTune &t, cudaEvent_t e0, cudaEvent_t e1) {
         enqueue(t, 1);
         IQM_CHECK_CUDA(cudaEventRecord(e0, ctx->stream));
         enqueue(t, 1);
@@ -133,24 +134,30 @@ struct iqm_batch_plan {
 
     // Coordinate search over the FSIM shapes: budget of an inverse-pass chunk, rows per CTA of
     // the inverse row pass.  A candidate must be 2% faster
-    // to replace the current choice.
+    // to replace the current choice, and is passed over where the memory for it is missing.
     void autotune_fsim() {
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         IQM_CHECK_CUDA(cudaEventCreate(&e0));
         IQM_CHECK_CUDA(cudaEventCreate(&e1));
         try {
-            iqm::FsimTune best{};
+            iqm::FsimTune best = tune;
             float best_ms = time_fsim(best, e0, e1);
+            const int usual_mb = best.chunk_mb;
             auto consider = [&](iqm::FsimTune t) {
-                const float ms = time_fsim(t, e0, e1);
-                if (ms < best_ms * 0.98f) {
-                    best_ms = ms;
-                    best = t;
+                try {
+                    const int asked_mb = t.chunk_mb;
+                    const float ms = time_fsim(t, e0, e1);
+                    if (t.chunk_mb == asked_mb && ms < best_ms * 0.98f) {
+                        best_ms = ms;
+                        best = t;
+                    }
+                } catch (const iqm::Error &e) {
+                    if (e.code != IQM_ENOMEM) throw;
                 }
             };
-            for (int mb : {80, 1280}) {
+            for (int mb : {usual_mb / 8, usual_mb * 2}) {
                 iqm::FsimTune t = best;
-                t.chunk_mb = mb;
+                t.chunk_mb = std::max(1, mb);
                 consider(t);
             }
             {
@@ -161,7 +168,7 @@ struct iqm_batch_plan {
             tune = best;
             char line[160];
             std::snprintf(line, sizeof(line), "fsim: chunk_mb=%d rows_per_cta=%d (%.3f ms per batch)",
-                          tune.chunk_mb ? tune.chunk_mb : 640, tune.rows_per_cta, double(best_ms));
+                          tune.chunk_mb, tune.rows_per_cta, double(best_ms));
             info += line;
         } catch (...) {
             cudaEventDestroy(e0);
@@ -248,7 +255,10 @@ IQM_API int iqm_batch_plan_create(iqm_ctx *ctx, int metric_mask, const iqm_pair 
         plan->enqueue(plan->tune);
         if (autotune && (metric_mask & IQM_METRIC_FSIM)) {
             plan->autotune_fsim();
-            plan->enqueue(plan->tune);  // buffers sized for the chosen shapes
+            // buffers sized for the chosen shapes, not for the largest that were tried
+            IQM_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
+            plan->scratch[1].release();
+            plan->enqueue(plan->tune);
         } else {
             plan->info += "fsim: default shapes";
         }
