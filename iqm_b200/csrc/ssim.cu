@@ -97,23 +97,37 @@ __device__ __forceinline__ int find_pair(const SsimPairDev *pairs, int n, int ti
     return lo;
 }
 
-// Deterministic pooling: the CTA's partial (FP64, fixed order) goes to
-// its tile slot; the last CTA of the pair to finish sums the pair's slots in a fixed order and
-// writes the mean (`count` pooled pixels).  `red` holds NTH/32 doubles of shared memory.
+// Pooled values are sums of four rows' in units of 2^-37: a tile's 2^12 of them, below 8 each, are a whole
+// number that FP64 holds.
+constexpr double POOL_UNITS = 137438953472.0;
+
+// Sum over the CTA, in a fixed order; valid in thread 0.  `red` holds NTH/32 values of 8 bytes.
+template <int NTH, class T>
+__device__ __forceinline__ T cta_sum(T v, double *red) {
+    T *part = reinterpret_cast<T *>(red);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    T s = 0;
+#pragma unroll
+    for (int i = 0; i < NTH / 32; i++) s += part[i];
+    return s;
+}
+
+// Deterministic pooling: the CTA's partial goes to its tile slot; the last CTA of the pair to finish sums the
+// pair's slots, in units (a pair's may pass 64 bits: the upper 40 and lower 24 bits of each tile's add up by
+// themselves) so that neither the cut into tiles nor their order matters, and writes the mean (`count` pooled
+// pixels).  Values that are no such numbers (too large, infinities and NaN) add up in FP64.
 template <int NTH>
 __device__ __forceinline__ void pool_tiles(double d, double *red, int *is_last, double *partials,
                                            unsigned *counters, double *scores, int pi, const SsimPairDev &P,
                                            int gt, double count) {
     const int tid = threadIdx.x;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
-    if ((tid & 31) == 0) red[tid >> 5] = d;
-    __syncthreads();
+    d = cta_sum<NTH>(d, red);
     if (tid == 0) {
-        double s = 0.0;
-#pragma unroll
-        for (int i = 0; i < NTH / 32; i++) s += red[i];
-        partials[gt] = s;
+        partials[gt] = d;
         __threadfence();
         const unsigned prev = atomicAdd(&counters[pi], 1u);
         *is_last = (prev == unsigned(P.ntiles - 1));
@@ -121,18 +135,23 @@ __device__ __forceinline__ void pool_tiles(double d, double *red, int *is_last, 
     __syncthreads();
     if (!*is_last) return;
     __threadfence();
-    double s = 0.0;
-    for (int i = tid; i < P.ntiles; i += NTH) s += __ldcg(&partials[P.tile_base + i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    __syncthreads();
-    if ((tid & 31) == 0) red[tid >> 5] = s;
-    __syncthreads();
+    long long hi = 0, lo = 0;
+    double other = 0.0;
+    for (int i = tid; i < P.ntiles; i += NTH) {
+        const double v = __ldcg(&partials[P.tile_base + i]);
+        if (fabs(v) <= 32768.0) {
+            const long long u = __double2ll_rn(v * POOL_UNITS);
+            hi += u >> 24;
+            lo += u & 0xffffff;
+        } else {
+            other += v;
+        }
+    }
+    hi = cta_sum<NTH>(hi, red);
+    lo = cta_sum<NTH>(lo, red);
+    other = cta_sum<NTH>(other, red);
     if (tid == 0) {
-        double tot = 0.0;
-#pragma unroll
-        for (int i = 0; i < NTH / 32; i++) tot += red[i];
-        scores[pi] = tot / count;
+        scores[pi] = (double(hi) * (16777216.0 / POOL_UNITS) + double(lo) / POOL_UNITS + other) / count;
         counters[pi] = 0u;  // ready for the next launch
     }
 }
@@ -238,11 +257,11 @@ __global__ void __launch_bounds__(NT, 4) ssim_kernel(SsimArgs args) {
 #pragma unroll
     for (int k = 0; k < K - 1; k++) am[k] = as[k] = make_float2(0.f, 0.f);
     float acc = 0.f;     // pooled SSIM of up to four rows
-    long long sum = 0;   // and of the strip, in units of 2^-26
+    long long sum = 0;   // and of the strip, in POOL_UNITS
     double other = 0.0;  // sums that are no such numbers: k1 or k2 of 0 over flat areas
     auto pool = [&] {
         if (pool_x) {
-            if (fabsf(acc) < 16.0f) sum += __float2int_rn(acc * 67108864.0f);
+            if (fabsf(acc) < 8.0f) sum += __float2ll_rn(acc * float(POOL_UNITS));
             else other += acc;
         }
         acc = 0.f;
@@ -349,8 +368,7 @@ __global__ void __launch_bounds__(NT, 4) ssim_kernel(SsimArgs args) {
         __syncthreads();
     }
     pool();
-    // Sums of these are exact in FP64 (up to 2^27 pixels), so their order does not matter.
-    pool_tiles<NT>(double(sum) * (1.0 / 67108864.0) + other, red, &is_last, args.partials, args.counters, args.scores, pi, P, gt,
+    pool_tiles<NT>(double(sum) * (1.0 / POOL_UNITS) + other, red, &is_last, args.partials, args.counters, args.scores, pi, P, gt,
                    double(W - 2 * R + 1) * double(H - 2 * R + 1));
 }
 
