@@ -22,11 +22,14 @@ struct Error {
     std::string msg;
 };
 
+// The error goes with the exception: left pending, it would fail the next call's launches.
 #define IQM_CHECK_CUDA(expr)                                                              \
     do {                                                                                  \
         cudaError_t e_ = (expr);                                                          \
-        if (e_ != cudaSuccess)                                                            \
+        if (e_ != cudaSuccess) {                                                          \
+            cudaGetLastError();                                                           \
             throw ::iqm::Error{IQM_ECUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)}; \
+        }                                                                                 \
     } while (0)
 
 #define IQM_REQUIRE(cond, text)                                   \
