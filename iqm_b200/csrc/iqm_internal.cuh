@@ -317,6 +317,15 @@ __device__ __forceinline__ float sqrt_approx(float x) {  // sqrt(x), x >= 0
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// sqrt(x) and 1 / x for normal x > 0 to within an ulp: one Newton step on the SFU's values
+__device__ __forceinline__ float sqrt_newton(float x) {
+    const float r = rsqrt_approx(x), y = x * r;
+    return fmaf(0.5f * r, fmaf(-y, y, x), y);
+}
+__device__ __forceinline__ float rcp_newton(float x) {
+    const float y = rcp_approx(x);
+    return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
 // sqrt(v) for v >= 0 as v * rsqrt(v); 0 for v = 0
 __device__ __forceinline__ float sqrt_nonneg(float v) { return v * rsqrt_approx(fmaxf(v, 1e-30f)); }
 // x^y for x >= 0: exp2(y log2 x) for x > 0; for x = 0 the values of pow(0, y): 0 for y > 0, 1 for

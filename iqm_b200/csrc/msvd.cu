@@ -92,24 +92,14 @@ __device__ __forceinline__ void load_block(const uint8_t *img, long long pitch, 
         for (int k = 0; k < 4; k++) c[q][k] = iqm::add2(c[q][k], iqm::dup2(-8388608.0f));
 }
 
-// sqrt(x) and 1 / x for normal x > 0 to within an ulp: one Newton step on the SFU's values
-__device__ __forceinline__ float sqrt_newton(float x) {
-    const float r = iqm::rsqrt_approx(x), y = x * r;
-    return fmaf(0.5f * r, fmaf(-y, y, x), y);
-}
-__device__ __forceinline__ float rcp_newton(float x) {
-    const float y = iqm::rcp_approx(x);
-    return fmaf(y, fmaf(-x, y, 1.0f), y);
-}
-
 // A Householder reflection I - beta v v' that takes a vector of squared norm nn and first element x0 to
 // (alpha, 0, ...): v is the vector with x0 - alpha in place of x0.  A vector of zeros is left as it is
 // (beta 0), which also covers vectors of rounding noise too small for the squares of FP32.
 __device__ __forceinline__ void reflection(float nn, float x0, float &alpha, float &beta) {
     const bool live = nn > 1e-30f;
-    const float norm = sqrt_newton(fmaxf(nn, 1e-30f));
+    const float norm = iqm::sqrt_newton(fmaxf(nn, 1e-30f));
     alpha = live ? -copysignf(norm, x0) : 0.0f;
-    beta = live ? rcp_newton(fmaf(fabsf(x0), norm, nn)) : 0.0f;
+    beta = live ? iqm::rcp_newton(fmaf(fabsf(x0), norm, nn)) : 0.0f;
 }
 
 // Step K of the bidiagonalisation: column K is reflected to its diagonal element d, then row K right of
@@ -282,7 +272,7 @@ __device__ __forceinline__ bool svd8_qd(float2 (&c)[8][4], float (&s)[8]) {
     qd_smallest<2>(z);
     z.q[0] += z.sigma;
 #pragma unroll
-    for (int i = 0; i < 8; i++) s[i] = z.q[i] > 1e-30f ? sqrt_newton(z.q[i]) : 0.0f;
+    for (int i = 0; i < 8; i++) s[i] = z.q[i] > 1e-30f ? iqm::sqrt_newton(z.q[i]) : 0.0f;
     return z.converged;
 }
 
