@@ -347,9 +347,11 @@ __global__ void __launch_bounds__(NT, 4) ssim_kernel(SsimArgs args) {
                 const float num = fmaf(0.5f, mu2.x - mu2.y, args.c1) * fmaf(0.5f, varu - varv, args.c2);
                 const float den = fmaf(0.5f, mu2.x + mu2.y, args.c1) * fmaf(0.5f, varu + varv, args.c2);
                 // den is about c1 c2 or more, but 0 is possible: k1 or k2 may be 0, and the variances round; inside
-                // the reciprocal's range, 2^-126 to 2^126, as long as c1 c2 is.  A rounded product, so that no path
-                // adds it unrounded to the pooled sum
-                const float ssim = __fmul_rn(num, iqm::rcp_approx(den));
+                // the reciprocal's range, 2^-126 to 2^126, as long as c1 c2 is.  One Newton step on the quotient
+                // (2 of some 130 instructions), so that equal numerator and denominator, identical images, give 1.
+                // Explicit operations, so that every path pools the same bits
+                const float r = iqm::rcp_approx(den), q = __fmul_rn(num, r);
+                const float ssim = __fmaf_rn(__fmaf_rn(-den, q, num), r, q);
                 if constexpr (decltype(plain)::value) {
                     acc += ssim;
                 } else {
