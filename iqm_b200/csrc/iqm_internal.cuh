@@ -59,12 +59,14 @@ struct DevBuf {
         cap = want;
         return ptr;
     }
-    // As get, but nullptr when that much memory is not free, without giving the present buffer back.
+    // As get, but nullptr when that much memory is not free, without giving the present buffer back.  Leaves some
+    // for what the driver allocates by itself: streams, kernels on their first launch, graphs.
     void *try_get(size_t bytes, cudaStream_t s) {
+        constexpr size_t kRoom = size_t(64) << 20;
         if (bytes <= cap) return ptr;
         size_t avail = 0, total = 0;
         IQM_CHECK_CUDA(cudaMemGetInfo(&avail, &total));
-        if (bytes + 256 > avail + cap) return nullptr;
+        if (bytes + kRoom > avail + cap) return nullptr;
         try {
             return get(bytes, s);
         } catch (const Error &e) {

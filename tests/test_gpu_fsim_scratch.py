@@ -103,3 +103,24 @@ def test_many_sizes_share_the_budget(fresh, autotune):
     assert np.array_equal(got, np.tile(want, (20, 1)))
     # the planes, a budget of at most 1280 MB, and 100 MB for the graph
     assert took <= 20 * sum(_plane_bytes(w * h) for w, h in sizes) + (1280 if autotune else 640) * MB + 100 * MB, took
+
+
+@pytest.mark.parametrize("mb", range(60, 400, 20))
+def test_scratch_leaves_room_for_streams_and_graphs(fresh, mb):
+    import torch
+    pairs = [synth.rgb_gain_pair(h, w, config=1, pair=i) for i, (w, h) in enumerate([(480, 270), (300, 256), (270, 270)])]
+    keep, items = _device_pairs(pairs, 8)
+    want = [_scores(fresh, items[i:i + 1])[0] for i in range(3)]
+    out = torch.zeros(2 * len(items), dtype=torch.float64, device="cuda")
+    filler = _fill_all_but(8 * _plane_bytes(270 * 480 + 300 * 256 + 270 * 270) // MB + 100 + mb)
+    try:
+        plan = iqm_b200.BatchPlan(fresh, iqm_b200.METRIC_FSIM, items, out.data_ptr(), autotune=False)
+        try:
+            plan.run()
+            fresh.synchronize()
+            got = out.cpu().numpy().reshape(-1, 2)
+        finally:
+            plan.close()
+    finally:
+        del filler
+    assert np.array_equal(got, np.tile(want, (8, 1)))
