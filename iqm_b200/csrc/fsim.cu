@@ -1160,20 +1160,33 @@ iqm::FsimPlan *get_plan(iqm_ctx *ctx, int w2, int h2) {
 
 struct Layout {
     size_t yiq, spec, spec2, T, planes, thr, partials, total;
+    size_t spec_pair;  // complex elements from one pair's spectra in spec2 to the next one's
 };
 
 // G pairs of the group; chunk pairs' worth of inverse-pass intermediates.
 // nbuf: inverse-pass intermediate buffers (2 when consecutive chunks alternate between two streams).
 // tiled: elements of a spectrum plane of the register engine (0: not used).
+// That engine's spectra take no memory of their own.  A pair's two lie in its amplitude planes, which only the
+// row pass after its column pass writes (all but planes narrower than a tile fit there); the packed ones lie in
+// the energy planes, and are read for the last time before the first of those.
 Layout layout_for(int G, int chunk, int n, int tiles, int nbuf, int tiled) {
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     Layout L{};
     size_t off = 0;
     L.yiq = off; off += al(sizeof(float) * size_t(G) * 6 * n);
-    L.spec = off; off += al(sizeof(float2) * size_t(G) * n);
-    L.spec2 = off; off += al(sizeof(float2) * size_t(G) * 2 * tiled);
     L.T = off; off += al(sizeof(float2) * size_t(nbuf) * chunk * 32 * n);
     L.planes = off; off += al(sizeof(float) * size_t(G) * 24 * n);
+    if (!tiled) {
+        L.spec = off; off += al(sizeof(float2) * size_t(G) * n);
+    } else {
+        L.spec = L.planes + sizeof(float) * size_t(G) * 8 * n;
+        L.spec2 = L.planes;
+        L.spec_pair = size_t(4) * n;
+        if (2 * size_t(tiled) > L.spec_pair) {
+            L.spec_pair = 2 * size_t(tiled);
+            L.spec2 = off; off += al(sizeof(float2) * size_t(G) * L.spec_pair);
+        }
+    }
     L.thr = off; off += al(sizeof(float) * size_t(G) * 8);
     L.partials = off; off += al(sizeof(double) * size_t(G) * tiles * 3);
     L.total = off;
@@ -1340,6 +1353,7 @@ void fsim_enqueue(iqm_ctx *ctx, const std::vector<iqm_pair> &pairs, int energy_m
         g.yiq = reinterpret_cast<float *>(base + Lc.yiq);
         g.spec = reinterpret_cast<float2 *>(base + Lc.spec);
         g.spec2 = reinterpret_cast<float2 *>(base + Lc.spec2);
+        g.spec_pair = Lc.spec_pair;
         g.lc = P->lc;
         g.tile = P->tile;
         g.tiled = P->tiled;

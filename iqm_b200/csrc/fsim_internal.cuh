@@ -43,7 +43,8 @@ struct FsimGroup {
     int w2, h2, n;
     float *yiq;     // G x 2 x 3 x n   (I, Q, Y)
     float2 *spec;   // G x n: per pair the spectrum of Y_img + i Y_ref
-    float2 *spec2;  // G x 2 x tiled: each image's own spectrum (register engine)
+    float2 *spec2;  // per pair, spec_pair apart, 2 x tiled: each image's own spectrum (register engine)
+    size_t spec_pair;
     int lc, tile, tiled;  // FsimPlan's
     float2 *T;      // chunk x 2 x 16 x n  (after the column pass of the inverse transform)
     float *amp;     // G x 8 x n       (img*4 + o)

@@ -29,7 +29,7 @@ fsim_inv_cols_reg(FsimGroup g, const __grid_constant__ RegFft F, int lc_) {
     extern __shared__ __align__(16) float2 sm[];  // matrices, spectrum tile, two filter tiles
     const int o = blockIdx.y, plane = blockIdx.z;  // plane: chunk-local pair*2 + img
     const int x0 = blockIdx.x << lc, w2 = g.w2;
-    const float2 *S = g.spec2 + (size_t(g.pair0) * 2 + plane) * g.tiled + size_t(blockIdx.x) * g.tile;
+    const float2 *S = g.spec2 + size_t(g.pair0 + (plane >> 1)) * g.spec_pair + size_t(plane & 1) * g.tiled + size_t(blockIdx.x) * g.tile;
     const float *H = g.filters + size_t(o * 4) * g.tiled + size_t(blockIdx.x) * g.tile;
     const unsigned s_tile = smem_addr(sm) + 8u * (((F.size << lc) + 1) & ~1), h_tile = s_tile + 8u * g.tile;
     copy_run(h_tile, H, 4 * g.tile);  // the plan's, not the previous kernel's

@@ -59,7 +59,7 @@ fsim_fwd_cols_reg(FsimGroup g, const __grid_constant__ RegFft F, int lc) {
         [&](int, int, int) { return [](int, unsigned p, float2 v) { sts2(p, make_float2(v.y, v.x)); }; });
     __syncthreads();
     const RegStep &last = F.st[F.nsteps - 1];
-    float2 *S1 = g.spec2 + size_t(pair) * 2 * g.tiled, *S2 = S1 + g.tiled;
+    float2 *S1 = g.spec2 + size_t(pair) * g.spec_pair, *S2 = S1 + g.tiled;
     for (int w = threadIdx.x; w < (h2 << lc); w += blockDim.x) {
         const int seq = w & ((1 << lc) - 1), y = w >> lc;
         if ((seq & (half - 1)) >= used) continue;

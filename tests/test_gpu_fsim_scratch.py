@@ -124,3 +124,21 @@ def test_scratch_leaves_room_for_streams_and_graphs(fresh, mb):
     finally:
         del filler
     assert np.array_equal(got, np.tile(want, (8, 1)))
+
+
+@pytest.mark.parametrize("w,h", [(300, 260), (20, 9), (7, 400), (2, 4096), (4096, 3)])
+def test_planes_hold_the_spectra(fresh, w, h):
+    """A pair takes 30 floats a point of its plane beside a chunk's, what the planes alone take, apart from planes
+    narrower than a tile of 8 columns; and planes of any width hold them (the score is a lone pair's)."""
+    import torch
+    pairs = [synth.rgb_gain_pair(h, w, config=1, pair=i) for i in range(3)]
+    count = max(3, int(3e9 / (120 * w * h)) // 3 * 3) if w >= 8 else 99
+    keep, items = _device_pairs(pairs, min(count, 30000) // 3)
+    want = [_scores(fresh, items[i:i + 1])[0] for i in range(3)]
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    got = _scores(fresh, items)
+    took = before - torch.cuda.mem_get_info()[0]
+    assert np.array_equal(got, np.tile(want, (len(items) // 3, 1)))
+    if w >= 8:  # 4% for the pooling sums of a tile, the descriptors and what is left of a tile of 256 points
+        assert took <= len(items) * (125 * w * h + 600) + 700 * MB, took
