@@ -208,8 +208,8 @@ struct Chunk {
 };
 
 // Bound by the FMA pipe and instruction issue: of the instructions a pixel pair takes, 47 are the packed taps
-// of both passes.  Four CTAs per SM at 126 registers, 16 1080p pairs: 213 us (236 us with a row's tests in
-// every row instead of once a step), against 397 us for the form before it (a column a thread, eleven loads and squares per pixel, the row loop
+// of both passes.  Four CTAs per SM at 125 registers, 16 1080p pairs: 214 us (236 us with a row's tests in
+// every row instead of once a step; a Newton step on the quotient for identical images' sake took 217), against 397 us for the form before it (a column a thread, eleven loads and squares per pixel, the row loop
 // unrolled over the window, a barrier a row; 297 instructions a pixel pair); five CTAs at 96 registers
 // spill, 253 us.  The split-precision tensor-core form took 23.1 us a 1080p pair and the single-product
 // one 15.6 us where this takes 13.3, so every form asked for computes here.
@@ -347,11 +347,11 @@ __global__ void __launch_bounds__(NT, 4) ssim_kernel(SsimArgs args) {
                 const float num = fmaf(0.5f, mu2.x - mu2.y, args.c1) * fmaf(0.5f, varu - varv, args.c2);
                 const float den = fmaf(0.5f, mu2.x + mu2.y, args.c1) * fmaf(0.5f, varu + varv, args.c2);
                 // den is about c1 c2 or more, but 0 is possible: k1 or k2 may be 0, and the variances round; inside
-                // the reciprocal's range, 2^-126 to 2^126, as long as c1 c2 is.  One Newton step on the quotient
-                // (2 of some 130 instructions), so that equal numerator and denominator, identical images, give 1.
-                // Explicit operations, so that every path pools the same bits
-                const float r = iqm::rcp_approx(den), q = __fmul_rn(num, r);
-                const float ssim = __fmaf_rn(__fmaf_rn(-den, q, num), r, q);
+                // the reciprocal's range, 2^-126 to 2^126, as long as c1 c2 is.  A rounded product, so that no path
+                // adds it unrounded to the pooled sum
+                float ssim = __fmul_rn(num, iqm::rcp_approx(den));
+                // equal numerator and denominator, as in identical images, make 1 without the reciprocal's error
+                if (num == den) ssim = rintf(ssim);
                 if constexpr (decltype(plain)::value) {
                     acc += ssim;
                 } else {
@@ -386,8 +386,10 @@ void launch_ssim(const SsimArgs &a, int total_tiles, cudaStream_t s) {
 // Rows of a tile, the same for all pairs of a launch: the power of two that divides SHIFT_ROWS with the
 // least estimated time, a tile's rows with its halo (and about a dozen rows' worth of set-up) times the
 // rounds of two CTAs per SM that it takes.  The values of an image do not depend on the choice.  Strips
-// of 8 / 16 / 32 / 64 / 128 rows: one 512x512 pair 15.2 / 15.5 / 19.6 / 27.5 / 43.5 us, 16 1080p pairs
-// 504 / 350 / 273 / 238 / 236 us (before steps without row tests, which took 236 to 213).
+// of 8 / 16 / 32 / 64 / 128 rows: one 512x512 pair 15.3 / 15.3 / 18.1 / 25.2 / 37.5 us, one 1080p pair
+// 42.0 / 31.8 / 29.8 / 29.7 / 38.0, four 131 / 92 / 74 / 66 / 71, 16 pairs 494 / 334 / 254 / 219 / 215 us.  Four
+// CTAs run on an SM, but rounds of one, two or four choose within 2% of one another there, but for four 1080p
+// pairs (71 / 71 / 66 us) and one of 720p (21.5 / 21.1 / 22.3 us).
 int strip_rows(const iqm_pair *pairs, int n, int R) {
     int best = SHIFT_ROWS;
     double best_cost = 0.0;
