@@ -25,6 +25,6 @@ def test_the_chain_is_found():
     assert len(list(_early_kernels())) >= 6
 
 
-@pytest.mark.parametrize("body", _early_kernels())
+@pytest.mark.parametrize("body", list(_early_kernels()))
 def test_no_read_only_loads(body):
     assert "__ldg(" not in body and "ld.global.nc" not in body
