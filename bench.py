@@ -56,10 +56,10 @@ TRAFFIC = {
     "ssim": {"kernel": "ssim_kernel", "bytes_per_launch": 137500000, "pairs_per_launch": 8},
     # fsim_inv_rows_reg, 8 pairs: 265.5 MB read + 72.3 MB written (profiles/fsim_inverse_passes.md)
     "fsim": {"kernel": "fsim_inv_rows_kernel", "bytes_per_launch": 337900000, "pairs_per_launch": 8},
-    # flip_kernel, 4 pairs: 67.8 MB read + 3.3 MB written (profiles/flip_kernel_1080p.md)
-    "flip": {"kernel": "flip_kernel", "bytes_per_launch": 71100000, "pairs_per_launch": 4},
-    # msvd_block_kernel, 8 pairs: 131.8 MB read + 3.8 MB written (profiles/msvd_block_kernel_1080p.md)
-    "msvd": {"kernel": "msvd_block_kernel", "bytes_per_launch": 135600000, "pairs_per_launch": 8},
+    # flip_kernel, 4 pairs: 67.8 MB read + 3.7 MB written (profiles/flip_kernel_1080p.md)
+    "flip": {"kernel": "flip_kernel", "bytes_per_launch": 71400000, "pairs_per_launch": 4},
+    # msvd_block_kernel, 8 pairs: 132.2 MB read + 6.7 MB written (profiles/msvd_block_kernel_1080p.md)
+    "msvd": {"kernel": "msvd_block_kernel", "bytes_per_launch": 138900000, "pairs_per_launch": 8},
 }
 
 

@@ -44,7 +44,9 @@ extern "C" {
 typedef struct iqm_ctx iqm_ctx;
 
 /* Least precision that a caller accepts.  The FP32 kernels are now also the fastest of every metric, so
- * all three values compute plain FP32 arithmetic with FP64 pooling sums. */
+ * all three values compute plain FP32 arithmetic.  Scores are pooled without a loss that FP64 would not have:
+ * FSIM and M-SVD sum in FP64, FLIP the map's values and SSIM the FP32 sums of four rows of them in whole numbers
+ * (of 2^-47 and 2^-37), which do not depend on how a picture is cut into tiles. */
 typedef enum {
     IQM_FP32 = 0,
     IQM_MIXED = 1,
@@ -87,7 +89,7 @@ int iqm_ssim(iqm_ctx *ctx, const uint8_t *rgba_in, const uint8_t *rgba_ref, int 
  * w*h floats), plus the stream to run on (NULL = the default stream); the call returns without
  * synchronising.  The kernel's scratch is a fixed array inside the library (about 33 KB) that every
  * GPU which loads the library holds until the process exits, so the image may span at most
- * IQM_SSIM_NOALLOC_MAX_TILES tiles of 128 columns x 122 rows (11-tap window; e.g. 7680x4320 uses
+ * IQM_SSIM_NOALLOC_MAX_TILES areas of 128 columns x 122 rows (11-tap window; e.g. 7680x4320 spans
  * 2160); larger images return IQM_EINVAL.  The first call on a device looks up that array's device
  * address with the device current, so make it before any stream capture.  The address is kept for
  * the device's primary context (the one the CUDA runtime uses): callers in other driver-API

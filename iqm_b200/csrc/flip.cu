@@ -763,7 +763,10 @@ FusedTaps fused_taps(const FlipTaps &T, int R) {
 
 // Output rows of a tile, the same for all pairs of a launch: whole steps of FROWS rows less the window's
 // 2 R, of the least estimated time (a tile's steps and a step's worth of set-up, times the rounds of two
-// CTAs per SM).  No value depends on the choice.
+// CTAs per SM, which is what fits up to radius 11; one does beyond).  No value depends on the choice.
+// Tiles of 4 / 6 / 8 / 10 / 12 steps at 67 pixels per degree: one 512x512 pair 37 / 48 / 61 / 73 / 85 us (chosen: 40),
+// one 1080p pair 139 / 123 / 129 / 109 / 128 (128), four 470 / 397 / 378 / 379 / 369 us (381); at 97, radius 13:
+// 45 / 45 / 57 / 67 / 80 (46), 201 / 164 / 152 / 164 / 152 (163), 779 / 595 / 534 / 521 / 498 us (498).
 int strip_rows(const std::vector<iqm_pair> &pairs, int R) {
     int best = 0;
     double best_cost = 0.0;

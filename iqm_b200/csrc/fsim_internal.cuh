@@ -70,9 +70,9 @@ __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontr
 // Launches a kernel that calls wait_for_previous(): its CTAs are set up during the tail of the stream's
 // previous kernel, which saves a launch latency per kernel of a chain of short ones.
 // carveout > 0: the share of the SM's array kept as shared memory, in percent.  early = false: after the
-// previous kernel's end as usual; so where chunks of pairs alternate between two streams, whose kernels already
-// fill each other's tails (32 1080p pairs 1002 us, with early launches 993; one 512x384 pair 73 us, with early
-// launches 58).
+// previous kernel's end as usual.  One 512x384 pair 73 us, with early launches 58.  Where chunks of pairs alternate
+// between two streams, whose kernels fill much of each other's tails, they are not used yet, though they gain
+// there as well: 32 1080p pairs 999.6 us, with early launches 985.6.
 template <class... Params, class... Args>
 inline void launch_after(void (*fn)(Params...), dim3 grid, int threads, size_t smem, int carveout, bool early, cudaStream_t st,
                          Args... args) {

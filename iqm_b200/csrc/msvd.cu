@@ -379,8 +379,8 @@ __device__ __forceinline__ void block_values(const MsvdArgs &args, const MsvdPai
 // Two lanes per block slot: the even lane takes the block of the distorted image, the odd lane the
 // same block of the reference; the odd lane's singular values reach the even lane by shuffle.  One
 // copy of the SVD code serves both images and twice as many blocks are in flight.
-// Bound by instruction issue (72% of the issue slots, FMA pipe 52%, 4.7k instructions a block of one
-// image, about a sixth of them lost to lanes that wait for their warp's slowest qd sweep).  16 1080p
+// Bound by instruction issue (78% of the issue slots, FMA pipe 54%, 5.0k instructions a warp of 16 blocks of both
+// images, some of them lost to lanes that wait for their warp's slowest qd sweep).  16 1080p
 // pairs: 475 us with Jacobi sweeps, 183 us now; five CTAs per SM at 93 registers took 185 us where six at 80
 // took 178 us.
 __global__ void __launch_bounds__(BLOCK_THREADS, 6) msvd_block_kernel(MsvdArgs args) {
